@@ -4,8 +4,8 @@
 ``fftm_b200/csrc`` with nvcc (``-gencode arch=compute_100a,code=sm_100a``) into
 objects under ``fftm_b200/_build`` and links ``fftm_b200/libfftb_b200.so``
 (CUDA runtime linked statically, so the library does not depend on the runtime
-version that other libraries in the process load).  The pass kernel is
-instantiated in 8 parts per precision so the compiler runs in parallel.
+version that other libraries in the process load).  The pass and line kernels are
+instantiated in parts so the compiler runs in parallel.
 """
 from __future__ import annotations
 
@@ -21,11 +21,12 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libfftb_b200.so")
-NPARTS = 8
+NPARTS = 8        # objects of the pass kernel's instantiations
+LINE_NPARTS = 16  # objects per precision of the line kernel's
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
-              "--expt-relaxed-constexpr", f"-DFFTB_NPARTS={NPARTS}"]
+NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xfatbin=--compress-mode=size", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
+              "--expt-relaxed-constexpr", f"-DFFTB_NPARTS={NPARTS}", f"-DFFTB_LINE_NPARTS={LINE_NPARTS}"]
 
 
 def nvcc() -> str:
@@ -79,9 +80,12 @@ def _jobs():
             continue
         src = os.path.join(CSRC, f)
         if f == "fftb_pass_inst.cu":
+            for k in range(NPARTS):
+                jobs.append((src, os.path.join(BUILD, f"pass_float_{k}.o"), ["-DFFTB_REAL=float", f"-DFFTB_PART={k}"]))
+        elif f == "fftb_line_inst.cu":
             for real in ("float", "double"):
-                for k in range(NPARTS):
-                    obj = os.path.join(BUILD, f"pass_{real}_{k}.o")
+                for k in range(LINE_NPARTS):
+                    obj = os.path.join(BUILD, f"line_{real}_{k}.o")
                     jobs.append((src, obj, [f"-DFFTB_REAL={real}", f"-DFFTB_PART={k}"]))
         else:
             jobs.append((src, os.path.join(BUILD, f[:-3] + ".o"), []))
@@ -92,7 +96,8 @@ def _jobs():
 def _compile(job, digest):
     src, obj, extra = job
     stamp = obj + ".stamp"
-    key = digest + "|" + " ".join(extra) + "|" + str(os.path.getmtime(src))
+    with open(src, "rb") as fh:  # by content: a copied tree keeps its objects
+        key = digest + "|" + " ".join(NVCC_FLAGS + extra) + "|" + hashlib.sha256(fh.read()).hexdigest()
     if os.path.exists(obj) and os.path.exists(stamp) and open(stamp).read() == key:
         return obj, None
     cmd = [nvcc()] + ARCH + NVCC_FLAGS + extra + ["-c", src, "-o", obj]

@@ -13,18 +13,17 @@
 
 #include "../../include/fftb.h"
 #include "fftb_device.cuh"
+#include "fftb_line.cuh"
 
-#ifndef FFTB_NPARTS
-#define FFTB_NPARTS 8
-#endif
-
-// Kernel tables exported by the fftb_pass_inst.cu objects.
-#define FFTB_DECL_PART(R, k) extern "C" int fftb_pass_table_##R##_part##k(fftb::PassKernelInfo *, int);
-#define FFTB_DECL_PARTS(R)                                                                                            \
-    FFTB_DECL_PART(R, 0) FFTB_DECL_PART(R, 1) FFTB_DECL_PART(R, 2) FFTB_DECL_PART(R, 3) FFTB_DECL_PART(R, 4)          \
-    FFTB_DECL_PART(R, 5) FFTB_DECL_PART(R, 6) FFTB_DECL_PART(R, 7)
-FFTB_DECL_PARTS(float)
-FFTB_DECL_PARTS(double)
+// Kernel tables exported by the fftb_pass_inst.cu and fftb_line_inst.cu objects.
+#define FFTB_DECL_PASS(k) extern "C" int fftb_pass_table_float_part##k(fftb::PassKernelInfo *, int);
+#define FFTB_DECL_LINE(k)                                                                                             \
+    extern "C" int fftb_line_table_float_part##k(fftb::LineKernelInfo *, int);                                        \
+    extern "C" int fftb_line_table_double_part##k(fftb::LineKernelInfo *, int);
+#define FFTB_PARTS8(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7)
+#define FFTB_PARTS16(X) FFTB_PARTS8(X) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15)
+FFTB_PARTS8(FFTB_DECL_PASS)
+FFTB_PARTS16(FFTB_DECL_LINE)
 
 namespace fftb {
 
@@ -33,28 +32,40 @@ namespace {
 thread_local std::string g_last_error;
 
 struct Registry {
-    std::map<int, PassKernelInfo> tab[2];
+    std::vector<PassKernelInfo> pass = std::vector<PassKernelInfo>(4097, PassKernelInfo{});  // f32 pass kernels by length
+    std::vector<LineKernelInfo> line[2];  // [2 length + row mapping], nf = 0 where there is none
     std::set<std::pair<int, const void *>> smem_configured;  // (device, kernel): the limit is per device
     std::map<std::tuple<int, int, int>, void *> roots;  // (device, dtype, ntw) -> device table
+    std::map<std::tuple<int, int, int, int>, void *> stages;  // (device, dtype, nf, row) -> stage tables
     std::mutex mu;
 
     Registry()
     {
-        typedef int (*part_fn)(PassKernelInfo *, int);
-        const part_fn f32[] = {fftb_pass_table_float_part0, fftb_pass_table_float_part1,
-                               fftb_pass_table_float_part2, fftb_pass_table_float_part3,
-                               fftb_pass_table_float_part4, fftb_pass_table_float_part5,
-                               fftb_pass_table_float_part6, fftb_pass_table_float_part7};
-        const part_fn f64[] = {fftb_pass_table_double_part0, fftb_pass_table_double_part1,
-                               fftb_pass_table_double_part2, fftb_pass_table_double_part3,
-                               fftb_pass_table_double_part4, fftb_pass_table_double_part5,
-                               fftb_pass_table_double_part6, fftb_pass_table_double_part7};
-        PassKernelInfo buf[256];
-        for (int d = 0; d < 2; ++d)
-            for (int p = 0; p < 8; ++p) {
-                const int n = (d == 0 ? f32[p] : f64[p])(buf, 256);
-                for (int i = 0; i < n && i < 256; ++i) tab[d][buf[i].nf] = buf[i];
+#define FFTB_FN_PASS(k) fftb_pass_table_float_part##k,
+#define FFTB_FN_LINE32(k) fftb_line_table_float_part##k,
+#define FFTB_FN_LINE64(k) fftb_line_table_double_part##k,
+        int (*const fp[])(PassKernelInfo *, int) = {FFTB_PARTS8(FFTB_FN_PASS)};
+        int (*const fl[2][16])(LineKernelInfo *, int) = {{FFTB_PARTS16(FFTB_FN_LINE32)}, {FFTB_PARTS16(FFTB_FN_LINE64)}};
+        PassKernelInfo pb[256];
+        for (auto f : fp) {
+            const int n = f(pb, 256);
+            for (int i = 0; i < n && i < 256; ++i)
+                if (pb[i].nf <= 4096) pass[pb[i].nf] = pb[i];
+        }
+        std::vector<LineKernelInfo> lb(256);
+        for (int d = 0; d < 2; ++d) {
+            line[d].resize(2 * 4097);
+            for (auto f : fl[d]) {
+                const int n = f(lb.data(), 256);
+                for (int i = 0; i < n && i < 256; ++i)
+                    if (lb[i].nf <= 4096) line[d][2 * lb[i].nf + lb[i].row] = lb[i];
             }
+        }
+    }
+    const LineKernelInfo *find_line(int dtype, int nf, int row) const
+    {
+        if (nf < 1 || nf > 4096 || line[dtype][2 * nf + row].nf != nf) return nullptr;
+        return &line[dtype][2 * nf + row];
     }
 };
 
@@ -109,6 +120,69 @@ int get_roots(int dtype, int ntw, void **out)
     return FFTB_SUCCESS;
 }
 
+// table w[(q - 1) ns + j] = exp(-2 pi i q j / (ns rad)), q = 1 .. rad - 1, j < ns
+template <typename R> __global__ void make_stage_kernel(cpx<R> *w, int ns, int rad)
+{
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m < (rad - 1) * ns) {
+        double s, c;
+        sincospi(-2.0 * (double)((m / ns + 1) * (m % ns)) / (double)(ns * rad), &s, &c);
+        w[m] = mk<R>((R)c, (R)s);
+    }
+}
+
+// The line kernel's stage tables (of its plan, then of the reversed plan), made once per device.
+int get_stages(int dtype, const LineKernelInfo &k, void **out)
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return set_status_from_cuda(e);
+    Registry &r = reg();
+    std::lock_guard<std::mutex> lk(r.mu);
+    auto key = std::make_tuple(dev, dtype, k.nf, k.row);
+    auto it = r.stages.find(key);
+    if (it != r.stages.end()) {
+        *out = it->second;
+        return FFTB_SUCCESS;
+    }
+    const LinePlan rev = line_reverse(k.plan);
+    const size_t n = (size_t)line_table_size(k.plan) + (size_t)line_table_size(rev);
+    if (n == 0) {
+        *out = nullptr;
+        return FFTB_SUCCESS;
+    }
+    char *p = nullptr;
+    e = cudaMalloc(&p, complex_bytes(dtype) * n);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        set_last_error("cudaMalloc of a stage table failed");
+        return FFTB_ERROR_ALLOC;
+    }
+    size_t base = 0;
+    for (const LinePlan &pl : {k.plan, rev}) {
+        int ns = 1;
+        for (int i = 0; i < pl.S; ++i) {
+            const int rad = pl.r[i], cnt = (rad - 1) * ns;
+            if (i > 0) {
+                char *w = p + complex_bytes(dtype) * (base + (size_t)line_tab_off(pl, i));
+                if (dtype == FFTB_F32) make_stage_kernel<float><<<(cnt + 255) / 256, 256>>>((float2 *)w, ns, rad);
+                else make_stage_kernel<double><<<(cnt + 255) / 256, 256>>>((double2 *)w, ns, rad);
+            }
+            ns *= rad;
+        }
+        base += (size_t)line_table_size(pl);
+    }
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e != cudaSuccess) {
+        cudaFree(p);
+        return set_status_from_cuda(e);
+    }
+    r.stages[key] = p;
+    *out = p;
+    return FFTB_SUCCESS;
+}
+
 long long labs_ll(long long v) { return v < 0 ? -v : v; }
 
 int floor_pow2(int v)
@@ -130,21 +204,32 @@ int set_status_from_cuda(cudaError_t e)
     return e == cudaErrorMemoryAllocation ? FFTB_ERROR_ALLOC : FFTB_ERROR_CUDA;
 }
 
-bool has_kernel(int dtype, int nf)
-{
-    Registry &r = reg();
-    return r.tab[dtype].count(nf) != 0;
-}
+bool has_kernel(int dtype, int nf) { return reg().find_line(dtype, nf, 1) != nullptr; }
 
 int engine_roots(int dtype, int ntw, void **out) { return get_roots(dtype, ntw, out); }
 
-bool lookup_kernel(int dtype, int nf, PassKernelInfo *out)
+bool lookup_kernel(int nf, PassKernelInfo *out)
 {
     Registry &r = reg();
-    auto it = r.tab[dtype].find(nf);
-    if (it == r.tab[dtype].end()) return false;
-    *out = it->second;
+    if (nf < 1 || nf > 4096 || r.pass[nf].nf != nf) return false;
+    *out = r.pass[nf];
     return true;
+}
+
+// Division by d of l < 2^31 as (l m) >> (31 + s): s = ceil(log2 d), m = ceil(2^(31+s) / d) < 2^32; the
+// product's excess l (m d - 2^(31+s)) is below 2^31 2^s, so the quotient is exact.
+void line_divisors(PassArgs &a)
+{
+    a.c_shift = -1;
+    if (a.nlines > 0x7fffffffLL) return;
+    auto magic = [](long long d, unsigned *m) {
+        int s = 0;
+        while ((1LL << s) < d) ++s;
+        *m = (unsigned)((((unsigned long long)1 << (31 + s)) + (unsigned long long)d - 1) / (unsigned long long)d);
+        return 31 + s;
+    };
+    const int s0 = magic(a.c0, &a.c0_mul), s1 = magic(a.c1, &a.c1_mul);
+    a.c_shift = s0 | (s1 << 6);
 }
 
 int program_add(Program &prog, int dtype, const AxisPass &p)
@@ -157,16 +242,16 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
     bool half = realk && (p.n % 2 == 0);
     int nf = half ? p.n / 2 : p.n;
     Registry &r = reg();
-    auto it = r.tab[dtype].find(nf);
-    if (it == r.tab[dtype].end() && half) {
+    bool line = r.find_line(dtype, nf, 1) != nullptr;
+    if (!line && half) {
         // no half-length kernel: the real line as a full complex line
         half = false;
         nf = p.n;
-        it = r.tab[dtype].find(nf);
+        line = r.find_line(dtype, nf, 1) != nullptr;
     }
     bool chirpz = false;
-    if (it != r.tab[dtype].end()) {
-        L.k = it->second;
+    if (line) {
+        if (!lookup_kernel(nf, &L.k)) L.k = PassKernelInfo{nf, 1, pad16(nf) + 1, nullptr};
     } else if (bluestein_kernel(dtype, p.n, &L.k)) {
         chirpz = true;   // L.k.nf is the convolution length
         const void *ch = nullptr, *bh = nullptr;
@@ -314,19 +399,41 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
     a.gshift = gs;
     L.block = G * T;
     L.smem = smem_of(G);
-    const long long ncta = (nlines + G - 1) / G;
+    long long ncta = (nlines + G - 1) / G;
+    L.fn = L.k.fn;
+    if (line) {
+        // the thread mapping follows the input side; a side of the other order, or with blocked
+        // points, is staged through shared memory
+        const LineKernelInfo &k = *r.find_line(dtype, nf, a.in_pts_fast ? 1 : 0);
+        if ((p.ep_mode & ~(EP_SCALE | EP_HALFW | EP_TWIDDLE)) != 0 && p.kind != K_SANDWICH) return FFTB_ERROR_INVALID_VALUE;
+        a.line_in = !p.in_blk && (!k.row || p.is == 1);
+        a.line_out = a.out_pts_fast == a.in_pts_fast && !p.out_blk && (!k.row || p.os == 1);
+        line_divisors(a);
+        void *tab = nullptr;
+        if ((st = get_stages(dtype, k, &tab)) != FFTB_SUCCESS) return st;
+        a.ltw = tab;
+        L.fn = p.kind == K_SANDWICH ? k.fn_sand : k.fn;
+        L.block = k.NT;
+        L.smem = a.line_in && a.line_out ? k.smem : k.smem_t;
+        ncta = (nlines + k.G - 1) / k.G;
+    }
     if (ncta > 0x7fffffffLL) return FFTB_ERROR_INVALID_VALUE;
     L.grid = dim3((unsigned)ncta, 1, 1);
     {
         std::lock_guard<std::mutex> lk(r.mu);
-        if (L.smem > 48 * 1024) {
+        if (L.smem > 40 * 1024) {  // beside up to 8 KB of static shared memory
             int dev = 0;
             cudaError_t e = cudaGetDevice(&dev);
             if (e != cudaSuccess) return set_status_from_cuda(e);
-            if (!r.smem_configured.count({dev, L.k.fn})) {
-                e = cudaFuncSetAttribute(L.k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+            if (!r.smem_configured.count({dev, L.fn})) {
+                // to what the device allows beside the kernel's static shared memory
+                cudaFuncAttributes fa;
+                e = cudaFuncGetAttributes(&fa, L.fn);
+                if (e == cudaSuccess)
+                    e = cudaFuncSetAttribute(L.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             227 * 1024 - (int)fa.sharedSizeBytes);
                 if (e != cudaSuccess) return set_status_from_cuda(e);
-                r.smem_configured.insert({dev, L.k.fn});
+                r.smem_configured.insert({dev, L.fn});
             }
         }
     }
@@ -341,7 +448,7 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
         const long long pin = (p.kind == K_C2R) ? (long long)(p.n / 2 + 1) : (long long)p.n;
         const long long pout = (p.kind == K_R2C) ? (long long)(p.n / 2 + 1) : (long long)p.n;
         L.alg_bytes = (double)nlines * ((double)pin * (double)in_el + (double)pout * (double)out_el);
-        L.name = std::string(chirpz ? "fftb_bluestein_kernel<" : "fftb_pass_kernel<") + (dtype == 0 ? "f32" : "f64") +
+        L.name = std::string(chirpz ? "fftb_bluestein_kernel<" : "fftb_line_kernel<") + (dtype == 0 ? "f32" : "f64") +
                  "," + std::to_string(chirpz ? L.k.nf : nf) + ">/" + kn[p.kind] + "/n" + std::to_string(p.n);
     }
     prog.dtype = dtype;
@@ -431,7 +538,7 @@ int program_exec(const Program &prog, void *in, void *out, void *work, cudaStrea
             if (ep->mode >= 0) a.ep_mode = ep->mode;
         }
         void *args[] = {&a};
-        cudaError_t e = cudaLaunchKernel(L.k.fn, L.grid, dim3(L.block), args, L.smem, stream);
+        cudaError_t e = cudaLaunchKernel(L.fn, L.grid, dim3(L.block), args, L.smem, stream);
         if (e != cudaSuccess) return set_status_from_cuda(e);
     }
     if (timer) return timer_end(timer, stream);

@@ -57,7 +57,8 @@ struct LongLine;
 
 struct Launch {
     PassArgs args;
-    PassKernelInfo k;
+    PassKernelInfo k;    // the pass kernel's tile of this length (the batch kernels run it)
+    const void *fn;      // the kernel this launch runs: the line kernel, or the chirp-z pass
     int in_buf, out_buf;
     size_t in_off_bytes, out_off_bytes;
     int pair_candidate;  // real side contiguous with even strides
@@ -111,10 +112,10 @@ int timer_end(LaunchTimer *t, cudaStream_t s);
 // device table of the forward roots exp(-2 pi i m / ntw), shared per (device, dtype, ntw)
 int engine_roots(int dtype, int ntw, void **out);
 
-// true if a line of complex length nf has a compiled kernel for dtype
+// true if a line of complex length nf has a line kernel for dtype
 bool has_kernel(int dtype, int nf);
-// copies the registry entry of the pass kernel for (dtype, nf); false if none
-bool lookup_kernel(int dtype, int nf, PassKernelInfo *out);
+// copies the registry entry of the f32 pass kernel of length nf; false if none
+bool lookup_kernel(int nf, PassKernelInfo *out);
 
 // element size of the complex type
 inline size_t complex_bytes(int dtype) { return dtype == 0 ? 8 : 16; }

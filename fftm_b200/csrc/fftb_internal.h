@@ -64,6 +64,14 @@ struct PassArgs {
     int in_blk, out_blk;
     long long in_hi, out_hi;
     void *out_peer[8];
+    // line kernel (fftb_line.cuh): its stage tables, and whether the input and output sides have the
+    // order of the kernel's thread mapping (0: that side is staged through shared memory)
+    const void *ltw;
+    int line_in, line_out;
+    // l / c0 = (l c0_mul) >> (c_shift & 63) and q / c1 = (q c1_mul) >> (c_shift >> 6) for l, q < 2^31
+    // (c_shift < 0: more lines than that, divide)
+    unsigned c0_mul, c1_mul;
+    int c_shift;
 };
 
 struct PassKernelInfo {

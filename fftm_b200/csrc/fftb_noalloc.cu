@@ -90,19 +90,25 @@ struct NaPass {
     double ep_scale, ep_sign;
 };
 
+bool has_pass(int nf)
+{
+    PassKernelInfo k;
+    return lookup_kernel(nf, &k);
+}
+
 int launch_pass(const NaPass &p, cudaStream_t stream)
 {
     const bool realk = (p.kind == K_R2C || p.kind == K_C2R);
     bool half = realk && (p.n % 2 == 0);
     int nf = half ? p.n / 2 : p.n;
     PassKernelInfo k;
-    if (half && !lookup_kernel(FFTB_F32, nf, &k)) {
+    if (half && !lookup_kernel(nf, &k)) {
         // no half-length kernel: the real line runs as a full complex line of length n,
         // as the regular pass programs do (its root table, [0], has length n)
         half = false;
         nf = p.n;
     }
-    if (!lookup_kernel(FFTB_F32, nf, &k)) return FFTB_ERROR_UNSUPPORTED_SIZE;
+    if (!lookup_kernel(nf, &k)) return FFTB_ERROR_UNSUPPORTED_SIZE;
     PassArgs a;
     memset(&a, 0, sizeof(a));
     a.in = p.in;
@@ -177,8 +183,8 @@ extern "C" int fftb_poisson3d_f32_noalloc(const float *rhs, float *solution, lon
     // every line length must have a pass kernel of its own (R2C/C2R of even nz run nz/2, or
     // nz as a full complex line when nz/2 has none); lengths that need the chirp-z passes do
     // not, since those need a padded work line of their own
-    const bool zok = has_kernel(FFTB_F32, (int)nz) || (nz % 2 == 0 && has_kernel(FFTB_F32, (int)(nz / 2)));
-    if (!zok || !has_kernel(FFTB_F32, (int)ny) || !has_kernel(FFTB_F32, (int)nx)) {
+    const bool zok = has_pass((int)nz) || (nz % 2 == 0 && has_pass((int)(nz / 2)));
+    if (!zok || !has_pass((int)ny) || !has_pass((int)nx)) {
         set_last_error("fftb_poisson3d_f32_noalloc: a line length has no direct pass kernel");
         return FFTB_ERROR_UNSUPPORTED_SIZE;
     }

@@ -19,8 +19,8 @@
 #define FFTB_CAT(a, b) FFTB_CAT2(a, b)
 #define FFTB_CAT4(a, b, c, d) FFTB_CAT(FFTB_CAT(a, b), FFTB_CAT(c, d))
 
-// The complex line lengths the engine supports directly (R2C/C2R of even n
-// run NF = n/2, everything else NF = n).
+// The complex line lengths of the pass kernel (R2C/C2R of even n run NF = n/2, everything else
+// NF = n).
 #define FFTB_NF_LIST(X)                                                                            \
     X(1) X(2) X(4) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096)            \
     X(3) X(6) X(12) X(24) X(48) X(96) X(192) X(384) X(768) X(1536) X(3072)                         \
