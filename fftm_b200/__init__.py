@@ -444,7 +444,7 @@ class ffts:
                "spectrum_truncate")
 
     def derivative(self, u, out, axis, stream=None):
-        """du/d(axis) of a periodic field on [0, 2 pi)^d (spectral, fused R2C / C2R)."""
+        """du/d(axis) of a periodic field on [0, 2 pi)^d (spectral, fused into the axis's own transform)."""
         self._ensure()
         self._bind(stream)
         _check(_lib.load().fftb_ffts_derivative(self._h, _ptr(u), _ptr(out), int(axis)), "derivative")

@@ -29,10 +29,6 @@ struct XColEp {
     float hw_f;
     double hw;
     int tc;  // host side: launch the tensor-core variant of the kernel
-    // EP_DERIV (3D, inverse mode): multiply by i k_daxis * dscale before the x FFT
-    int daxis;
-    float dscale_f;
-    double dscale;
 };
 
 template <int NX> struct XColShape {
@@ -130,19 +126,7 @@ __device__ __forceinline__ void xcol_multiply(cpx<R> (&v)[16], int t, int cg0, c
     const R kyz = R(ky * ky + kz * kz + kw * kw);
     const R sc = sizeof(R) == 4 ? R(ep.scale_f) : R(ep.scale);
     const R sg = sizeof(R) == 4 ? R(ep.sign_f) : R(ep.sign);
-    if (ep.mode & EP_DERIV) {
-        // i k v * scale with k = kx (row), ky or kz (the column); 3D only.  kz is the half
-        // axis: its Nyquist bin carries the real cosine part, whose derivative the C2R
-        // drops with the imaginary part, the same as a separate multiply does
-        const R ds = sizeof(R) == 4 ? R(ep.dscale_f) : R(ep.dscale);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            const int kxi = t + T * j;
-            const int k = ep.daxis == 0 ? (kxi <= NX / 2 ? kxi : kxi - NX) : (ep.daxis == 1 ? ky : kz);
-            const R fct = R(k) * ds;
-            v[j] = mk<R>(-fct * v[j].y, fct * v[j].x);
-        }
-    } else if ((ep.mode & (EP_POISSON | EP_GAUSS)) == EP_POISSON) {
+    if ((ep.mode & (EP_POISSON | EP_GAUSS)) == EP_POISSON) {
         const R ss = sc * sg;
         const R tr = R(t);
 #pragma unroll
@@ -185,8 +169,7 @@ template <typename R> __device__ __forceinline__ void xcol_halfw(cpx<R> (&v)[16]
     }
 }
 
-// MODE 0: forward, 1: inverse, 2: forward -> spectral multiply -> inverse (in place, or
-// into tdata, laid out like data, when tdata is given),
+// MODE 0: forward, 1: inverse, 2: forward -> spectral multiply -> inverse, in place;
 // 3: forward, written transposed: column col becomes the contiguous row tout[col][kx],
 // 4: inverse of 3: reads the rows tin[col][kx], writes the columns in place of `data`.
 // blockIdx.y selects a batch of column sets `bstride` elements apart (the transposed
@@ -254,9 +237,8 @@ __device__ __forceinline__ void xcol_tile(cpx<R> *__restrict__ data, long long s
             dstp[(size_t)rr * NX + kx] = scr[rr * RP + kx];
         }
     } else if (ok) {
-        C *q = (MODE == 2 && tdata) ? tdata + (size_t)batch * bstride + cg0 : p;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) q[(size_t)(t + T * j) * stride] = v[j];
+        for (int j = 0; j < 16; ++j) p[(size_t)(t + T * j) * stride] = v[j];
     }
 }
 

@@ -249,6 +249,10 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
         nf = p.n;
         line = r.find_line(dtype, nf, 1) != nullptr;
     }
+    if ((p.ep_mode & EP_DERIV) && (!line || (p.kind != K_C2R && p.kind != K_SANDWICH))) {
+        set_last_error("the derivative multiply needs a line kernel");
+        return FFTB_ERROR_UNSUPPORTED_SIZE;
+    }
     bool chirpz = false;
     if (line) {
         if (!lookup_kernel(nf, &L.k)) L.k = PassKernelInfo{nf, 1, pad16(nf) + 1, nullptr};
@@ -405,7 +409,7 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
         // the thread mapping follows the input side; a side of the other order, or with blocked
         // points, is staged through shared memory
         const LineKernelInfo &k = *r.find_line(dtype, nf, a.in_pts_fast ? 1 : 0);
-        if ((p.ep_mode & ~(EP_SCALE | EP_HALFW | EP_TWIDDLE)) != 0 && p.kind != K_SANDWICH) return FFTB_ERROR_INVALID_VALUE;
+        if ((p.ep_mode & ~(EP_SCALE | EP_HALFW | EP_TWIDDLE | EP_DERIV)) != 0 && p.kind != K_SANDWICH) return FFTB_ERROR_INVALID_VALUE;
         a.line_in = !p.in_blk && (!k.row || p.is == 1);
         a.line_out = a.out_pts_fast == a.in_pts_fast && !p.out_blk && (!k.row || p.os == 1);
         line_divisors(a);

@@ -659,8 +659,7 @@ __device__ __forceinline__ void xcol_fft_regtw(cpx<R> (&v)[16], cpx<R> *scr, con
 template <typename R, int NX, int MODE>
 __global__ void __launch_bounds__(256, 2)
     xcol_ring_kernel(const __grid_constant__ CUtensorMap tmap, cpx<R> *__restrict__ data, long long stride,
-                     int ncols, int tpb, int ntiles, long long bstride, cpx<R> *__restrict__ tdata,
-                     const cpx<R> *__restrict__ roots, XColEp ep)
+                     int ncols, int tpb, int ntiles, long long bstride, const cpx<R> *__restrict__ roots, XColEp ep)
 {
     using C = cpx<R>;
     constexpr int T = XColShape<NX>::T, W = XColShape<NX>::W;
@@ -729,7 +728,7 @@ __global__ void __launch_bounds__(256, 2)
         }
         if (MODE != 2 && (ep.mode & EP_HALFW)) xcol_halfw<R>(v, cg0, ep);
         if (cg0 < ncols) {
-            C *q = ((MODE == 2 && tdata) ? tdata : data) + (size_t)b * bstride + cg0;
+            C *q = data + (size_t)b * bstride + cg0;
 #pragma unroll
             for (int j = 0; j < 16; ++j) q[(size_t)(t + T * j) * stride] = v[j];
         }
@@ -930,11 +929,10 @@ int device_sms()
 
 // The persistent TMA-ring column kernel takes modes 0-2 of a 16-byte aligned spectrum whose
 // row and batch pitches are multiples of 16 bytes (the tensor map's stride rule).
-bool ring_eligible(int mode, const void *data, long long stride, long long nbatch, long long bstride,
-                   const void *tdata, const XColEp &x)
+bool ring_eligible(int mode, const void *data, long long stride, long long nbatch, long long bstride, const XColEp &x)
 {
     if (mode > 2 || x.tc || getenv("FFTB_DISABLE_RING")) return false;
-    if ((uintptr_t)data % 16 || (tdata && (uintptr_t)tdata % 16)) return false;
+    if ((uintptr_t)data % 16) return false;
     if ((stride * 8) % 16 || (nbatch > 1 && (bstride * 8) % 16)) return false;
     return true;
 }
@@ -956,7 +954,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 }
 
 int launch_xcol_ring(const XColEntry *e, int mode, void *data, long long stride, long long ncols, long long nbatch,
-                     long long bstride, void *tdata, void *roots, XColEp x, cudaStream_t s)
+                     long long bstride, void *roots, XColEp x, cudaStream_t s)
 {
     const int W = 256 / (e->nx / 16);
     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
@@ -980,10 +978,9 @@ int launch_xcol_ring(const XColEntry *e, int mode, void *data, long long stride,
     const long long tpb = (ncols + W - 1) / W, ntiles = tpb * nbatch;
     const long long ctas = std::min<long long>(ntiles, 2LL * device_sms());
     float2 *d = (float2 *)data;
-    float2 *td = (float2 *)tdata;
     int nc = (int)ncols, tp = (int)tpb, nt = (int)ntiles;
     const float2 *rt = (const float2 *)roots;
-    void *args[] = {&map, &d, &stride, &nc, &tp, &nt, &bstride, &td, &rt, &x};
+    void *args[] = {&map, &d, &stride, &nc, &tp, &nt, &bstride, &rt, &x};
     return set_status_from_cuda(
         cudaLaunchKernel(e->fn_ring[mode], dim3((unsigned)ctas), dim3(256), args, e->smem_ring, s));
 }
@@ -993,7 +990,7 @@ int launch_xcol_n(const XColEntry *e, int mode, void *data, long long stride, lo
                   long long bstride, void *tdata, void *roots, XColEp x, cudaStream_t s, LaunchTimer *tm)
 {
     const int W = 256 / (e->nx / 16);
-    const bool ring = ring_eligible(mode, data, stride, nbatch, bstride, tdata, x);
+    const bool ring = ring_eligible(mode, data, stride, nbatch, bstride, x);
     if (tm) {
         static const char *mn[] = {"fwd", "inv", "sandwich", "fwd_t", "inv_t"};
         int st = timer_mark(tm, s,
@@ -1002,7 +999,7 @@ int launch_xcol_n(const XColEntry *e, int mode, void *data, long long stride, lo
                             (double)e->nx * ncols * nbatch * 16.0);
         if (st != FFTB_SUCCESS) return st;
     }
-    if (ring) return launch_xcol_ring(e, mode, data, stride, ncols, nbatch, bstride, tdata, roots, x, s);
+    if (ring) return launch_xcol_ring(e, mode, data, stride, ncols, nbatch, bstride, roots, x, s);
     float2 *d = (float2 *)data;
     float2 *td = (float2 *)tdata;
     int nc = (int)ncols;
@@ -1235,59 +1232,6 @@ int fused3d_spectral(const Fused3D &f, const void *in, void *out, void *work, co
     if (st == FFTB_SUCCESS) st = launch_xcol(f, 2, work, &ep, s, t);
     if (st == FFTB_SUCCESS)
         st = launch_plane(f, true, work, out, 1.0 / (double)(f.nx * f.ny * f.nz), s, t);
-    if (st == FFTB_SUCCESS && t) st = timer_end(t, s);
-    return st;
-}
-
-// du/d(axis): plane R2C into spec, the x column sandwich (forward, i k, inverse) in place,
-// the inverse planes with 1/N
-int fused3d_derivative(const Fused3D &f, const void *in, void *spec, void *out, int axis, cudaStream_t s,
-                       LaunchTimer *t)
-{
-    const long long nzh = f.nz / 2 + 1;
-    int st = launch_plane(f, false, in, spec, 1.0, s, t);
-    if (st == FFTB_SUCCESS) {
-        XColEp x = make_ep(nullptr);
-        x.mode = EP_DERIV;
-        x.daxis = axis;
-        x.dscale = 1.0;
-        x.dscale_f = 1.f;
-        x.nzh = (int)nzh;
-        x.ny = (int)f.ny;
-        x.nz = (int)f.nz;
-        x.hn = (int)f.nz;
-        x.tc = f.tc ? 1 : 0;
-        st = launch_xcol_n((const XColEntry *)f.xcol, 2, spec, f.ny * nzh, f.ny * nzh, 1, 0, nullptr, f.roots_x, x, s,
-                           t);
-    }
-    if (st == FFTB_SUCCESS) st = launch_plane(f, true, spec, out, 1.0 / (double)(f.nx * f.ny * f.nz), s, t);
-    if (st == FFTB_SUCCESS && t) st = timer_end(t, s);
-    return st;
-}
-
-// every first derivative: the planes' R2C once into spec; per axis the column sandwich
-// with the i k multiply from spec into spec2 and the inverse planes into outs[axis]
-int fused3d_gradient(const Fused3D &f, const void *in, void *spec, void *spec2, void *const *outs, cudaStream_t s,
-                     LaunchTimer *t)
-{
-    const long long nzh = f.nz / 2 + 1;
-    int st = launch_plane(f, false, in, spec, 1.0, s, t);
-    for (int a = 0; a < 3 && st == FFTB_SUCCESS; ++a) {
-        XColEp x = make_ep(nullptr);
-        x.mode = EP_DERIV;
-        x.daxis = a;
-        x.dscale = 1.0;
-        x.dscale_f = 1.f;
-        x.nzh = (int)nzh;
-        x.ny = (int)f.ny;
-        x.nz = (int)f.nz;
-        x.hn = (int)f.nz;
-        x.tc = f.tc ? 1 : 0;
-        st = launch_xcol_n((const XColEntry *)f.xcol, 2, spec, f.ny * nzh, f.ny * nzh, 1, 0, spec2, f.roots_x, x, s,
-                           t);
-        if (st == FFTB_SUCCESS)
-            st = launch_plane(f, true, spec2, outs[a], 1.0 / (double)(f.nx * f.ny * f.nz), s, t);
-    }
     if (st == FFTB_SUCCESS && t) st = timer_end(t, s);
     return st;
 }

@@ -36,12 +36,6 @@ int fused3d_spectral(const Fused3D &f, const void *in, void *out, void *work, co
                      LaunchTimer *t);
 int fused3d_forward_adjoint(const Fused3D &f, void *gspec, void *greal, cudaStream_t s, LaunchTimer *t);
 int fused3d_backward_adjoint(const Fused3D &f, const void *greal, void *gspec, cudaStream_t s, LaunchTimer *t);
-// du/d(axis) (0 = x, 1 = y, 2 = z) through the spectrum buffer spec: 3 launches
-int fused3d_derivative(const Fused3D &f, const void *in, void *spec, void *out, int axis, cudaStream_t s,
-                       LaunchTimer *t);
-// all three first derivatives: 7 launches, the spectrum written once and read per axis
-int fused3d_gradient(const Fused3D &f, const void *in, void *spec, void *spec2, void *const *outs, cudaStream_t s,
-                     LaunchTimer *t);
 int fused3d_num_launches(const Fused3D &f, int which);
 
 // The x or y FFTs of many f32 3D spectra [nx][ny][nz/2+1] of one line length in one launch,

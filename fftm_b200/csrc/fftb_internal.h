@@ -22,7 +22,7 @@ enum EpMode : int {
     EP_POISSON = 2,  // multiply by ep_sign / |k|^2 (0 at k = 0)
     EP_GAUSS = 4,    // multiply by exp(-|k|^2 * ep_gauss)
     EP_HALFW = 8,    // multiply interior bins of the half (R2C) axis by ep_hw (adjoint weights)
-    EP_DERIV = 16,   // multiply by i k_axis * scale (spectral derivative; fused column kernel)
+    EP_DERIV = 16,   // multiply by i k of the lines' own axis (spectral derivative: a sandwich, or the load of a C2R)
     EP_TWIDDLE = 32, // multiply output point p by w_L^(p j), j the batch index of ep_src[0], L = ep_n[0]
                      // (the inter-step twiddle of a four-step long line; w from the table ep_tw)
 };

@@ -563,6 +563,9 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
     // Z[N-k] = conj(E - i O) with E = X[k] + conj X[N-k], O = (X[k] - conj X[N-k]) conj(w_2N^k), DC and
     // Nyquist counted with their real parts.  Each pair is read once and goes through the
     // exchange area to the threads that start the transform.
+    // EP_DERIV multiplies bin b by i b first (the derivative along a half axis).
+    const bool drv = !SAND && (a.ep_mode & EP_DERIV);
+    auto times_ik = [](int k, C x) -> C { return mk<R>(-R(k) * x.y, R(k) * x.x); };
     auto load_packed = [&](bool stage, const C *x, long long st) {
         C xa[PH], xb[PH];
         const C *pa = x + t * st, *pb = x + (N - t) * st;
@@ -571,6 +574,13 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
             const bool ok = i + 1 < PH || t + T * i <= N / 2;
             xa[i] = ok ? *pa : mk<R>(R(0), R(0));
             xb[i] = ok ? *pb : mk<R>(R(0), R(0));
+        }
+        if (drv) {
+#pragma unroll
+            for (int i = 0; i < PH; ++i) {
+                xa[i] = times_ik(t + T * i, xa[i]);
+                xb[i] = times_ik(N - t - T * i, xb[i]);
+            }
         }
         if (stage) __syncthreads();  // every line is read before the packed ones overwrite them
         const C *tw = reinterpret_cast<const C *>(a.tw) + t;
@@ -594,6 +604,7 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
     };
     // full line of a half spectrum: bin p from x, which holds bin p or (p > N/2) bin N - p
     auto extend = [&](int p, C x) -> C {
+        if (drv) x = times_ik(p <= N / 2 ? p : N - p, x);
         if (p > N / 2) x = cconj(x);
         if (p == 0 || 2 * p == N) x.y = R(0);
         return x;
@@ -669,6 +680,8 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
                 const R k2 = fac.k2(p);
                 return cscale(z, k2 == R(0) ? R(0) : ss / k2);
             });
+        else if (a.ep_mode & EP_DERIV)  // i k along the lines' own full axis, the Nyquist bin at +n/2
+            multiply([&](int p, C z) { return cscale(times_ik(p <= N / 2 ? p : p - N, z), sc); });
         else
             multiply([&](int, C z) { return cscale(z, sc); });
         line_stages<R, N, ROW, true, 0>(v, ln, tab + line_table_size(P), t);

@@ -124,3 +124,35 @@ def test_strided_points_and_lines(F, torch_cuda):
     got = out.cpu().numpy().reshape(lines, n, 3)
     assert rel(got[..., 0], np.fft.fft(x[..., 0].astype(np.complex128))) <= TOL["float32"]
     assert not got[..., 1:].any()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("dims,layout4", [((12, 20), None), ((9, 15), None), ((20, 18, 25), None), ((7, 64, 32), None),
+                                          ((64, 64, 64), None), ((17, 12, 10), None), ((6, 10, 8, 12), "pencil"),
+                                          ((6, 10, 8, 9), "slab"), ((8, 6, 10, 12), "native_xzwy")])
+def test_derivatives_of_one_axis(F, torch_cuda, dims, layout4, dtype):
+    """derivative() and gradient() (one axis's transform; (17, ...) takes the whole transform, as a
+    chirp-z axis does) against i k on numpy's half spectrum: k = index on the half axis and up to
+    n/2 on the full axes, the Nyquist bin at +n/2, the C2R keeping the real part of the half
+    axis's DC and Nyquist bins.  The multiply raises the rounding of the largest k by n/2 over
+    the mean k: four times the transform's tolerance."""
+    torch = torch_cuda
+    rng = np.random.default_rng(11)
+    u = rng.uniform(-1, 1, dims).astype(np.float32 if dtype == "float32" else np.float64)
+    d = len(dims)
+    spec = np.fft.rfftn(u.astype(np.float64))
+    f = F.ffts(dtype, strategy_4d=layout4 or "pencil").init(*dims)
+    arr = np.ascontiguousarray(u.T) if layout4 == "pencil" else u
+    x = torch.from_numpy(arr).cuda()
+    outs = [torch.empty_like(x) for _ in dims]
+    f.gradient(x, outs)
+    one = torch.empty_like(x)
+    for axis, n in enumerate(dims):
+        i = np.arange(n // 2 + 1 if axis == d - 1 else n)
+        k = np.where(i <= n // 2, i, i - n).reshape([-1 if a == axis else 1 for a in range(d)])
+        y = np.fft.ifftn(1j * k * spec, axes=tuple(range(d - 1)))
+        ref = np.fft.irfft(y, n=dims[-1], axis=d - 1)
+        f.derivative(x, one, axis)
+        for got in (outs[axis], one):
+            g = got.cpu().numpy()
+            assert rel(g.T if layout4 == "pencil" else g, ref) <= 4 * TOL[dtype], axis
