@@ -275,6 +275,8 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
         if (st != FFTB_SUCCESS) return st;
         Launch S;
         memset(&S.args, 0, sizeof(S.args));
+        S.fn = nullptr;
+        S.programmatic = 0;
         S.in_buf = p.in_buf;
         S.out_buf = p.out_buf;
         S.in_off_bytes = S.out_off_bytes = 0;
@@ -405,6 +407,7 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
     L.smem = smem_of(G);
     long long ncta = (nlines + G - 1) / G;
     L.fn = L.k.fn;
+    L.programmatic = line ? 1 : 0;
     if (line) {
         // the thread mapping follows the input side; a side of the other order, or with blocked
         // points, is staged through shared memory
@@ -542,7 +545,17 @@ int program_exec(const Program &prog, void *in, void *out, void *work, cudaStrea
             if (ep->mode >= 0) a.ep_mode = ep->mode;
         }
         void *args[] = {&a};
-        cudaError_t e = cudaLaunchKernel(L.fn, L.grid, dim3(L.block), args, L.smem, stream);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = L.grid;
+        cfg.blockDim = dim3(L.block);
+        cfg.dynamicSmemBytes = L.smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = L.programmatic ? 1 : 0;
+        cudaError_t e = cudaLaunchKernelExC(&cfg, L.fn, args);
         if (e != cudaSuccess) return set_status_from_cuda(e);
     }
     if (timer) return timer_end(timer, stream);
