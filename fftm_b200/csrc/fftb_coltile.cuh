@@ -176,8 +176,8 @@ template <typename R> __device__ __forceinline__ void xcol_halfw(cpx<R> (&v)[16]
 // side has NX * ncols elements per batch).
 // The body of one column tile (blockIdx.x of xcol_kernel): tile `tile` of batch `batch`.
 template <typename R, int NX, int MODE, bool TC>
-__device__ __forceinline__ void xcol_tile(cpx<R> *__restrict__ data, long long stride, int ncols, long long bstride,
-                                          cpx<R> *__restrict__ tdata, const cpx<R> *__restrict__ roots,
+__device__ __forceinline__ void xcol_tile(cpx<R> *data, long long stride, int ncols, long long bstride,
+                                          cpx<R> *tdata, const cpx<R> *__restrict__ roots,
                                           const XColEp &ep, int tile, int batch)
 {
     using C = cpx<R>;

@@ -46,6 +46,15 @@ namespace fftb {
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;\n" ::: "memory"); }
 
+// Programmatic launch: lets the next kernel's CTAs start (they wait here too) and waits for the whole
+// of the kernel before this one.  Every kernel below calls it before its first access to a
+// buffer, and takes its buffers without __restrict__: a load that the compiler may treat as
+// constant for the kernel's lifetime could be moved above the wait or served from a stale line.
+__device__ __forceinline__ void programmatic_wait()
+{
+    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;\n" ::: "memory");
+}
+
 constexpr int kRingWaitLimit = 1 << 22;  // polls of a bounded bulk-copy wait (seconds)
 __device__ int g_ring_wait_error;        // set when a bounded wait gave up (a copy never completed)
 
@@ -136,7 +145,7 @@ template <int NY, int NZ, int CL> using PlaneShape = PlaneShapeT<NY, NZ, CL, pla
 
 template <typename R, int NY, int NZ, int CL>
 __global__ void __launch_bounds__(PlaneShape<NY, NZ, CL>::NT, PlaneShape<NY, NZ, CL>::MINB_FWD)
-    plane_fwd_kernel(const R *__restrict__ in, cpx<R> *__restrict__ out, const cpx<R> *__restrict__ roots)
+    plane_fwd_kernel(const R *in, cpx<R> *out, const cpx<R> *__restrict__ roots)
 {
     using C = cpx<R>;
     using S = PlaneShape<NY, NZ, CL>;
@@ -163,6 +172,7 @@ __global__ void __launch_bounds__(PlaneShape<NY, NZ, CL>::NT, PlaneShape<NY, NZ,
         for (int q = 0; q < CL; ++q) dst[q] = cg::this_cluster().map_shared_rank(plane, (unsigned)q);
     }
     if constexpr (CL > 1) cluster_wait();  // every peer's shared memory exists from here on
+    programmatic_wait();
 
     // ---- stage z: R2C of this CTA's rows (two rows per complex FFT), pushed to the slot owners
     {
@@ -331,7 +341,7 @@ __global__ void __launch_bounds__(PlaneShape<NY, NZ, CL>::NT, PlaneShape<NY, NZ,
 
 template <typename R, int NY, int NZ, int CL>
 __global__ void __launch_bounds__(PlaneShape<NY, NZ, CL>::NT, PlaneShape<NY, NZ, CL>::MINB_INV)
-    plane_inv_kernel(const cpx<R> *__restrict__ in, R *__restrict__ out, const cpx<R> *__restrict__ roots, R scale)
+    plane_inv_kernel(const cpx<R> *in, R *out, const cpx<R> *__restrict__ roots, R scale)
 {
     using C = cpx<R>;
     using S = PlaneShape<NY, NZ, CL>;
@@ -352,6 +362,7 @@ __global__ void __launch_bounds__(PlaneShape<NY, NZ, CL>::NT, PlaneShape<NY, NZ,
     }
     const C *iplane = in + (size_t)x * NY * (NZ / 2 + 1);
     if constexpr (CL > 1) cluster_wait();  // every peer's shared memory exists from here on
+    programmatic_wait();
 
     // ---- stage y, one CTA per plane: the plane's spectrum rows [NY][NZ/2+1] are contiguous in
     // global memory with the pitch of rowsm, so one bulk copy brings the whole plane in (no
@@ -582,10 +593,10 @@ __global__ void __launch_bounds__(PlaneShape<NY, NZ, CL>::NT, PlaneShape<NY, NZ,
 }
 
 template <typename R, int NX, int MODE, bool TC>
-__global__ void __launch_bounds__(256, 3) xcol_kernel(cpx<R> *__restrict__ data, long long stride, int ncols,
-                                                   long long bstride, cpx<R> *__restrict__ tdata,
-                                                   const cpx<R> *__restrict__ roots, XColEp ep)
+__global__ void __launch_bounds__(256, 3) xcol_kernel(cpx<R> *data, long long stride, int ncols, long long bstride,
+                                                   cpx<R> *tdata, const cpx<R> *__restrict__ roots, XColEp ep)
 {
+    programmatic_wait();
     xcol_tile<R, NX, MODE, TC>(data, stride, ncols, bstride, tdata, roots, ep, (int)blockIdx.x, (int)blockIdx.y);
 }
 
@@ -658,7 +669,7 @@ __device__ __forceinline__ void xcol_fft_regtw(cpx<R> (&v)[16], cpx<R> *scr, con
 // `bstride` complex entries), box {2W, NX, 1}.  Tile k = (batch k / tpb, column block k % tpb).
 template <typename R, int NX, int MODE>
 __global__ void __launch_bounds__(256, 2)
-    xcol_ring_kernel(const __grid_constant__ CUtensorMap tmap, cpx<R> *__restrict__ data, long long stride,
+    xcol_ring_kernel(const __grid_constant__ CUtensorMap tmap, cpx<R> *data, long long stride,
                      int ncols, int tpb, int ntiles, long long bstride, const cpx<R> *__restrict__ roots, XColEp ep)
 {
     using C = cpx<R>;
@@ -689,6 +700,7 @@ __global__ void __launch_bounds__(256, 2)
         mbar_init_fence();
     }
     __syncthreads();
+    programmatic_wait();
     if (tid == 0)
         for (int q = 0; q < kRingStages; ++q)
             if (blockIdx.x + q * gridDim.x < (unsigned)ntiles) issue(q, blockIdx.x + q * gridDim.x);
@@ -848,6 +860,16 @@ int configure(const void *fn, size_t smem)
     return set_status_from_cuda(e);
 }
 
+int device_sms()
+{
+    static int sms[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        sms[dev] = 148;
+    return sms[dev];
+}
+
 // One launch of a plane kernel over `nplanes` planes.
 int launch_plane_n(const PlaneEntry *e, long long nplanes, bool inverse, const void *in, void *out, void *roots,
                    double scale, cudaStream_t s, LaunchTimer *tm)
@@ -859,15 +881,23 @@ int launch_plane_n(const PlaneEntry *e, long long nplanes, bool inverse, const v
     cfg.blockDim = dim3(e->nt);
     cfg.dynamicSmemBytes = inverse ? e->smem_inv : e->smem_fwd;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     cfg.attrs = attr;
-    cfg.numAttrs = 0;
+    cfg.numAttrs = 1;
+    // The inverse planes start early only when they fill at least half of the CTA slots that their
+    // shared memory leaves: fewer of them would pile up on the few SMs that the column kernel
+    // leaves free (128^3 Poisson back to back: 25.8 us as plain launches, 28.5 with every kernel
+    // programmatic, 22.6 with this rule; 64x256x256, 256 of 296 slots: 46.2, 39.1, 39.1; 256x64x64,
+    // 256 of 740: 18.6, 19.2, 17.4; 64^4 native round trip 181 -> 170; 64^3 20.5 -> 16.8)
+    const long long slots = (long long)device_sms() * (227 * 1024 / (long long)(e->smem_inv + 1024));
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = !inverse || 2 * nplanes * e->cl >= slots;
     if (e->cl > 1) {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = e->cl;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.numAttrs = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = e->cl;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
     }
     const double bytes = (double)nplanes * e->ny * (4.0 * e->nz + 8.0 * (e->nz / 2 + 1));
     if (tm) {
@@ -917,16 +947,6 @@ XColEp make_ep(const EpValues *ep)
     return x;
 }
 
-int device_sms()
-{
-    static int sms[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        sms[dev] = 148;
-    return sms[dev];
-}
-
 // The persistent TMA-ring column kernel takes modes 0-2 of a 16-byte aligned spectrum whose
 // row and batch pitches are multiples of 16 bytes (the tensor map's stride rule).
 bool ring_eligible(int mode, const void *data, long long stride, long long nbatch, long long bstride, const XColEp &x)
@@ -951,6 +971,22 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
             fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
     });
     return fn;
+}
+
+// a launch of a kernel that begins with programmatic_wait()
+cudaError_t launch_programmatic(const void *fn, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
 int launch_xcol_ring(const XColEntry *e, int mode, void *data, long long stride, long long ncols, long long nbatch,
@@ -982,7 +1018,7 @@ int launch_xcol_ring(const XColEntry *e, int mode, void *data, long long stride,
     const float2 *rt = (const float2 *)roots;
     void *args[] = {&map, &d, &stride, &nc, &tp, &nt, &bstride, &rt, &x};
     return set_status_from_cuda(
-        cudaLaunchKernel(e->fn_ring[mode], dim3((unsigned)ctas), dim3(256), args, e->smem_ring, s));
+        launch_programmatic(e->fn_ring[mode], dim3((unsigned)ctas), dim3(256), args, e->smem_ring, s));
 }
 
 // One launch of a column kernel: ncols columns `stride` apart per batch, nbatch batches.
@@ -1006,8 +1042,8 @@ int launch_xcol_n(const XColEntry *e, int mode, void *data, long long stride, lo
     const float2 *rt = (const float2 *)roots;
     void *args[] = {&d, &stride, &nc, &bstride, &td, &rt, &x};
     const dim3 grid((unsigned)((ncols + W - 1) / W), (unsigned)nbatch);
-    return set_status_from_cuda(cudaLaunchKernel(x.tc ? e->fn_tc[mode] : e->fn[mode], grid, dim3(256), args,
-                                                 x.tc ? e->smem_tc : e->smem, s));
+    return set_status_from_cuda(launch_programmatic(x.tc ? e->fn_tc[mode] : e->fn[mode], grid, dim3(256), args,
+                                                    x.tc ? e->smem_tc : e->smem, s));
 }
 
 int launch_xcol(const Fused3D &f, int mode, void *data, const EpValues *ep, cudaStream_t s, LaunchTimer *tm)
