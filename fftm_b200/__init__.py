@@ -75,10 +75,21 @@ def _ptr(t) -> int:
     return t.data_ptr()
 
 
+_current_raw_stream = None
+
+
 def _stream_ptr(stream=None) -> int:
-    torch = _torch()
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    """The raw stream of a call: ``stream``, or torch's current stream of the current device.
+    Taken without building a Stream object where torch has the raw accessor (1.1 us less a call)."""
+    global _current_raw_stream
+    if stream is not None:
+        return stream.cuda_stream
+    if _current_raw_stream is None:
+        torch = _torch()
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        device = torch.cuda.current_device
+        _current_raw_stream = (lambda: raw(device())) if raw else (lambda: torch.cuda.current_stream().cuda_stream)
+    return _current_raw_stream()
 
 
 def version() -> str:
@@ -115,6 +126,7 @@ class Plan:
                                 batch, ctypes.byref(h), ctypes.byref(ws))
         _check(st, "fftb_plan_create")
         self._h = h
+        self._stream = 0  # the stream the handle is bound to
         self.work_size = ws.value
 
     def __del__(self):
@@ -127,7 +139,10 @@ class Plan:
         self._h = None
 
     def set_stream(self, stream=None):
-        _check(_lib.load().fftb_plan_set_stream(self._h, _stream_ptr(stream)), "set_stream")
+        s = _stream_ptr(stream)
+        if s != self._stream:  # the handle keeps its stream between calls
+            _check(_lib.load().fftb_plan_set_stream(self._h, s), "set_stream")
+            self._stream = s
 
     def set_work_area(self, tensor_or_ptr):
         ptr = tensor_or_ptr if isinstance(tensor_or_ptr, int) else _ptr(tensor_or_ptr)
@@ -303,6 +318,7 @@ class ffts:
         self.dtype = _dtype_code(dtype)
         self.strategy_4d = _STRATEGY[strategy_4d]
         self._h = None
+        self._stream = 0  # the stream the handle is bound to
         self._dims = None
         self._work = None
 
@@ -372,7 +388,10 @@ class ffts:
         _check(_lib.load().fftb_ffts_set_work_area(self._h, _ptr(tensor)), "set_work_area")
 
     def _bind(self, stream):
-        _check(_lib.load().fftb_ffts_set_stream(self._h, _stream_ptr(stream)), "set_stream")
+        s = _stream_ptr(stream)
+        if s != self._stream:  # the handle keeps its stream between calls
+            _check(_lib.load().fftb_ffts_set_stream(self._h, s), "set_stream")
+            self._stream = s
 
     def forward(self, real_in, complex_out, stream=None):
         self._ensure(real_in.dim() if real_in.dim() in (2, 3, 4) else None)
