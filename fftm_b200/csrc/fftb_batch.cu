@@ -19,6 +19,13 @@
 // The grouped form runs the same items as one plain launch per (stage, line length)
 // group, each a kernel specialised for its length, in stream order (no waits), and
 // can be replayed from a CUDA graph the same way.
+//
+// Both run the line kernel's tiles (fftb_line.cuh), and row-pair tiles for the z rows of 64 points and
+// more.  512 uneven round trips (axes of 32 to 128 points): grouped 2403 -> 1995 us, persistent 3841
+// -> 3526 us against pass-kernel rows and the fused path's column tiles; per group, 96-point rows
+// 206 -> 128 us, 48-point 108 -> 64, 96-point columns 119 -> 100, 96- and 128-point x sandwiches
+// 131 -> 96 and 174 -> 144.  What bounds it now: the rows, 3.4-4.6 TB/s, by shared-memory and L1
+// wavefronts (64-byte segments of a row per group of eight threads).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,7 +39,7 @@
 #include "fftb_coltile.cuh"
 #include "fftb_engine.h"
 #include "fftb_fused3d.h"
-#include "fftb_pass.cuh"
+#include "fftb_line.cuh"
 
 namespace fftb {
 namespace {
@@ -50,13 +57,11 @@ struct PassBind {
     int in_buf, out_buf;
     long long in_off, out_off;  // bytes
     int nf;
-    // the tile form of a pass on the fused path's kernels (f32): 0 the pass kernel's tile;
-    // 1 a column tile (ckind 0-2 x forward / inverse / sandwich, 3-4 y forward / inverse) of
-    // n-point lines; 2 a row-pair tile of n-point z rows (ckind 0 R2C, 1 C2R)
-    int fast, ckind, n;
-    int lines, ny, nz;      // column: lines of the spectrum, its ny and nz; row: rows
-    float scale, sign;      // row C2R scale; column sandwich scale and Poisson sign
-    int ep_mode;            // column sandwich multiply
+    int lkind;                  // line tile of the pass: 0 rows, 1 columns, 2 column sandwich
+    // pair = 1 (f32 z rows of 64, 128 and 256 points): a tile of row pairs instead, dir 0 R2C, 1 C2R,
+    // of `lines` rows of n points, the C2R times scale
+    int pair, dir, n, lines;
+    float scale;
     const float2 *roots;    // n-point root table
 };
 
@@ -69,30 +74,8 @@ __device__ __forceinline__ int ld_acquire(const int *p)
 
 #define FFTB_BATCH_NF_LIST(X) X(8) X(12) X(16) X(20) X(24) X(32) X(40) X(48) X(64) X(80) X(96) X(128) X(160) X(192) X(256)
 
-// Column and row-pair tiles of the persistent launch, one non-inlined function per kind and
-// length (their own register allocation, as the pass tiles have).
-template <int N, int KIND> __device__ __noinline__ void batch_col_tile(const PassBind *b, void *data, int tile)
-{
-    if constexpr (KIND <= 2) {
-        XColEp ep = {};
-        ep.mode = b->ep_mode;
-        ep.scale_f = b->scale;
-        ep.sign_f = b->sign;
-        ep.scale = b->scale;
-        ep.sign = b->sign;
-        ep.ny = b->ny;
-        ep.nz = b->nz;
-        ep.nzh = b->nz / 2 + 1;
-        ep.hn = b->nz;
-        ep.hw_f = 1.f;
-        ep.hw = 1.0;
-        xcol_tile<float, N, KIND, false>(reinterpret_cast<float2 *>(data), b->lines, b->lines, 0, nullptr, b->roots, ep,
-                                         tile, 0);
-    } else {
-        const XGroupItem it{0, b->lines, tile, b->ny, b->nz};
-        ycol_tile<N, KIND - 3>(it, reinterpret_cast<float2 *>(data), b->roots);
-    }
-}
+// Row-pair tile of the persistent launch, one non-inlined function per direction and length (their
+// own register allocation, as the line tiles have).
 template <int N, int DIR>
 __device__ __noinline__ void batch_row_tile(const PassBind *b, const void *in, void *out, int tile)
 {
@@ -100,18 +83,18 @@ __device__ __noinline__ void batch_row_tile(const PassBind *b, const void *in, v
     row_tile<N, DIR>(it, in, out, b->roots);
 }
 
-#define FFTB_BATCH_COL_LIST(X) X(32) X(48) X(64) X(96) X(128) X(256)
 #define FFTB_BATCH_ROW_LIST(X) X(64) X(128) X(256)
 
-// One tile of a pass of line length NF; not inlined, so every length keeps its own
-// register allocation instead of the union of all of them.  The tile stages its lines
-// with cp.async: thread 0's acquire load of the producer counters followed by the
-// CTA barrier orders these loads after the producers' fenced stores (PTX memory model).
-template <int NF>
-__device__ __noinline__ void batch_tile(const PassArgs *a, const void *in, void *out, long long line0,
+// One line tile of a pass of line length NF (lkind as in PassBind); not inlined, so every length
+// and kind keeps its own register allocation instead of the union of all of them.  Thread 0's
+// acquire load of the producer counters followed by the CTA barrier orders its loads after the
+// producers' fenced stores (PTX memory model).
+template <int NF, int LKIND>
+__device__ __noinline__ void batch_tile(const PassArgs *a, const void *in, void *out, long long tile,
                                         unsigned char *smem)
 {
-    pass_body<float, NF, false, false>(*a, in, out, line0, smem);
+    static_assert(LineShape<float, NF, LKIND == 0>::NT <= kBatchThreads, "a tile fits the batch kernels' blocks");
+    line_body<float, NF, LKIND == 0, LKIND == 2, true>(*a, in, out, tile, smem, nullptr);
 }
 
 // ctl[0]: queue head, ctl[1]: error flag, ctl[2 + p]: finished tiles of pass p
@@ -164,23 +147,8 @@ __global__ void __launch_bounds__(kBatchThreads)
         const void *bufs[3] = {in, out, work};
         const void *pin = (const char *)bufs[b.in_buf] + b.in_off;
         void *pout = (char *)const_cast<void *>(bufs[b.out_buf]) + b.out_off;
-        const long long line0 = (long long)bi.tile * a->G;
-        if (b.fast == 1) {
-            void *data = const_cast<void *>(pin);
-            switch (b.n * 8 + b.ckind) {
-#define FFTB_CCASE(n)                                                                                                 \
-    case n * 8 + 0: batch_col_tile<n, 0>(&binds[bi.pass], data, bi.tile); break;                                     \
-    case n * 8 + 1: batch_col_tile<n, 1>(&binds[bi.pass], data, bi.tile); break;                                     \
-    case n * 8 + 2: batch_col_tile<n, 2>(&binds[bi.pass], data, bi.tile); break;                                     \
-    case n * 8 + 3: batch_col_tile<n, 3>(&binds[bi.pass], data, bi.tile); break;                                     \
-    case n * 8 + 4: batch_col_tile<n, 4>(&binds[bi.pass], data, bi.tile); break;
-                FFTB_BATCH_COL_LIST(FFTB_CCASE)
-#undef FFTB_CCASE
-            default:
-                break;
-            }
-        } else if (b.fast == 2) {
-            switch (b.n * 2 + b.ckind) {
+        if (b.pair) {
+            switch (b.n * 2 + b.dir) {
 #define FFTB_RCASE(n)                                                                                                 \
     case n * 2 + 0: batch_row_tile<n, 0>(&binds[bi.pass], pin, pout, bi.tile); break;                                 \
     case n * 2 + 1: batch_row_tile<n, 1>(&binds[bi.pass], pin, pout, bi.tile); break;
@@ -190,11 +158,11 @@ __global__ void __launch_bounds__(kBatchThreads)
                 break;
             }
         } else {
-            switch (b.nf) {
+            switch (b.nf * 4 + b.lkind) {
 #define FFTB_CASE(n)                                                                                                  \
-    case n:                                                                                                           \
-        batch_tile<n>(a, pin, pout, line0, smem_raw);                                                                 \
-        break;
+    case n * 4 + 0: batch_tile<n, 0>(a, pin, pout, bi.tile, smem_raw); break;                                         \
+    case n * 4 + 1: batch_tile<n, 1>(a, pin, pout, bi.tile, smem_raw); break;                                         \
+    case n * 4 + 2: batch_tile<n, 2>(a, pin, pout, bi.tile, smem_raw); break;
                 FFTB_BATCH_NF_LIST(FFTB_CASE)
 #undef FFTB_CASE
             default:
@@ -218,26 +186,27 @@ __device__ __forceinline__ const void *batch_buf(int k, const void *in, void *ou
     return k == 0 ? in : (k == 1 ? (const void *)out : (const void *)work);
 }
 
-template <int NF>
-__global__ void __launch_bounds__(kBatchThreads)
+template <int NF, int LKIND>
+__global__ void __launch_bounds__(kBatchThreads, 4)
     batch_group_kernel(const BatchItem *__restrict__ items, const PassArgs *__restrict__ passes,
                        const PassBind *__restrict__ binds, const void *in, void *out, void *work)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const BatchItem bi = items[blockIdx.x];
-    const PassArgs &a = passes[bi.pass];
     const PassBind b = binds[bi.pass];
     const void *pin = (const char *)batch_buf(b.in_buf, in, out, work) + b.in_off;
     void *pout = (char *)const_cast<void *>(batch_buf(b.out_buf, in, out, work)) + b.out_off;
-    pass_body<float, NF, false, false>(a, pin, pout, (long long)bi.tile * a.G, smem_raw);
+    line_body<float, NF, LKIND == 0, LKIND == 2, true>(passes[bi.pass], pin, pout, bi.tile, smem_raw, nullptr);
 }
 
-const void *batch_group_fn(int nf)
+const void *batch_group_fn(int nf, int lkind)
 {
     switch (nf) {
 #define FFTB_CASE(n)                                                                                                  \
     case n:                                                                                                           \
-        return (const void *)&batch_group_kernel<n>;
+        return lkind == 0   ? (const void *)&batch_group_kernel<n, 0>                                                 \
+               : lkind == 1 ? (const void *)&batch_group_kernel<n, 1>                                                 \
+                            : (const void *)&batch_group_kernel<n, 2>;
         FFTB_BATCH_NF_LIST(FFTB_CASE)
 #undef FFTB_CASE
     default:
@@ -272,13 +241,6 @@ cudaError_t raise_smem_limit(const void *fn)
     return e;
 }
 
-int floor_pow2(int v)
-{
-    int p = 1;
-    while (p * 2 <= v) p *= 2;
-    return p;
-}
-
 enum BatchOp { OP_FORWARD = 0, OP_BACKWARD = 1, OP_ROUNDTRIP = 2, OP_POISSON = 3, OP_COUNT = 4 };
 
 struct OpPlan {
@@ -298,20 +260,13 @@ struct OpPlan {
     struct Group {
         int offset, count, nf;
         size_t smem;
-        // x and y stages of lengths with a column kernel: one grouped column-kernel launch
-        // over count tiles (XGroupItem offset ..) instead of the pass items
-        bool xcol = false;
+        int lkind = 0;        // line tiles: PassBind's
         bool zrow = false;    // z stage as one grouped row-pair launch (RowGroupItem offset ..)
-        int in_buf = B_IN, out_buf = B_OUT;
-        int ckind = 0;        // col_group kind: 0/1/2 x forward / inverse / sandwich, 3/4 y
-        int buf = B_WORK;     // the buffer holding the spectra (in place)
+        int in_buf = B_IN, out_buf = B_OUT, dir = 0;
         void *roots = nullptr;
-        int ep_mode = 0;      // the sandwich's multiply (the pass epilogue)
-        double ep_scale = 1.0, ep_sign = -1.0;
     };
     std::vector<Group> groups;
     BatchItem *d_gitems = nullptr;
-    XGroupItem *d_xitems = nullptr;
     RowGroupItem *d_ritems = nullptr;
     // CUDA graph of the persistent launch (mode 2) or of the grouped launches (mode 4)
     cudaGraph_t graph = nullptr;
@@ -336,7 +291,7 @@ struct fftb_batch_s {
     void *work = nullptr;
     bool own_work = false;
     cudaStream_t stream = 0;
-    int tiles_scale = 1;                      // autotune knob: tiles of G/tiles_scale lines
+    int tiles_scale = 1;                      // autotune knob (the line tiles have one size: no effect)
     int ctas_per_sm = 0;                      // autotune knob: 0 = occupancy limit
     long long wait_limit = kSpinLimit;        // polls of a dependency wait before the error flag
 };
@@ -428,23 +383,13 @@ int build_plan(fftb_batch_s *b, int op, double sign)
     std::vector<int> deps(P.npasses, -1), ntiles(P.npasses, 0);
     size_t smem = 0;
     std::vector<size_t> pass_smem(P.npasses, 0);
-    // per stage: the column kind (x passes step C3 = ny * nzh between points, y passes nzh) or
-    // the z direction (R2C of contiguous real rows, scaled C2R back to them) of the stages the
-    // fused path's tiles can run (f32, in place for the column stages); the same for every
-    // transform, taken from the first
-    std::vector<int> st_ckind(P.nstages, -1), st_zdir(P.nstages, -1);
+    // per stage: the direction of the z stages that the row-pair tiles can run (f32 R2C of contiguous
+    // real rows, scaled C2R back to them); the same for every transform, taken from the first
+    std::vector<int> st_zdir(P.nstages, -1);
     for (int s = 0; s < P.nstages; ++s) {
         const Launch &L0 = P.seq.launches[tpass[0][s]];
         const PassArgs &a0 = L0.args;
         if (b->dtype != FFTB_F32 || L0.longline != nullptr || a0.bs_n != 0) continue;
-        const long long ny0 = b->dims[1], nzh0 = b->dims[2] / 2 + 1;
-        const bool inplace = L0.in_buf == L0.out_buf && L0.in_off_bytes == L0.out_off_bytes;
-        if (inplace && ny0 > 1) {
-            if (a0.kind == K_SANDWICH && a0.is == ny0 * nzh0) st_ckind[s] = 2;
-            else if ((a0.kind == K_C2C_FWD || a0.kind == K_C2C_INV) && a0.ep_mode == 0)
-                st_ckind[s] = a0.is == ny0 * nzh0 ? (a0.kind == K_C2C_FWD ? 0 : 1)
-                                                  : (a0.is == nzh0 ? (a0.kind == K_C2C_FWD ? 3 : 4) : -1);
-        }
         if (a0.half && a0.is == 1 && a0.os == 1) {
             if (a0.kind == K_R2C && a0.ep_mode == 0) st_zdir[s] = 0;
             else if (a0.kind == K_C2R && (a0.ep_mode & ~EP_SCALE) == 0) st_zdir[s] = 1;
@@ -460,17 +405,13 @@ int build_plan(fftb_batch_s *b, int op, double sign)
     for (int p = 0; p < P.npasses; ++p) {
         const Launch &L = P.seq.launches[p];
         PassArgs a = L.args;
-        const int T = L.k.threads_per_line;
-        if (!batch_nf_supported(L.k.nf) || a.bs_n != 0) P.persistent_ok = false;  // chirp-z lines: sequential
-        int G = std::min(a.G, floor_pow2(std::max(1, kBatchThreads / T)));
-        G = std::max(1, G / b->tiles_scale);
-        a.G = G;
-        int gs = 0;
-        while ((1 << gs) < G) ++gs;
-        a.gshift = gs;
+        // line tiles of 256 threads; chirp-z, long and other lengths: sequential only
+        const bool tiled = batch_nf_supported(L.k.nf) && L.line && a.line_in && a.line_out &&
+                           !(L.line->row && a.kind == K_SANDWICH);
+        if (!tiled) P.persistent_ok = false;
+        const int G = L.line ? L.line->G : a.G;
         a.pair_io = L.pair_candidate ? 1 : 0;  // buffers are 16-byte aligned (checked at execution)
-        const size_t cb = complex_bytes(b->dtype);
-        const size_t sm = (a.tw_smem ? (size_t)a.ntw * cb : 0) + (size_t)G * 32 + (size_t)G * L.k.line_pitch * cb;
+        const size_t sm = L.line ? L.line->smem : 0;
         smem = std::max(smem, sm);
         pass_smem[p] = sm;
         args[p] = a;
@@ -480,52 +421,27 @@ int build_plan(fftb_batch_s *b, int op, double sign)
         pb.in_off = (long long)L.in_off_bytes;
         pb.out_off = (long long)L.out_off_bytes;
         pb.nf = L.k.nf;
+        pb.lkind = a.kind == K_SANDWICH ? 2 : (L.line && L.line->row ? 0 : 1);
         ntiles[p] = (int)((a.nlines + G - 1) / G);
-        // the fused path's tile for this pass, where the stage has one for this length
+        // the row-pair tile, where it is the faster one (row_group_tile_pairs)
         const int st = stage_of[p], ti = trans_of[p];
-        const long long nx = b->dims[3 * ti], ny = b->dims[3 * ti + 1], nz = b->dims[3 * ti + 2];
         const int FZ = st_zdir[st] >= 0 ? row_group_tile_pairs(b->dtype, 2 * L.k.nf) : 0;
-        const int W = FZ == 0 && st_ckind[st] >= 0 ? col_group_tile_lines(b->dtype, L.k.nf) : 0;
-        void *roots = nullptr;
-        // the kernels' set-up (shared-memory limit, root table) once per kind and length
-        auto prepared = [&](int key, auto prepare) -> int {
-            auto it = roots_of.find(key);
-            if (it != roots_of.end()) {
-                roots = it->second;
-                return FFTB_SUCCESS;
-            }
-            int rs = prepare();
-            if (rs == FFTB_SUCCESS) roots_of[key] = roots;
-            return rs;
-        };
         if (FZ > 0) {
-            int rs = prepared(100000 + st_zdir[st] * 1000 + 2 * L.k.nf,
-                              [&] { return row_group_prepare(b->dtype, st_zdir[st], 2 * L.k.nf, &roots); });
-            if (rs != FFTB_SUCCESS) return rs;
-            pb.fast = 2;
-            pb.ckind = st_zdir[st];
+            // its set-up (shared-memory limit, root table) once per direction and length
+            void *&roots = roots_of[st_zdir[st] * 100000 + 2 * L.k.nf];
+            if (!roots) {
+                int rs = row_group_prepare(b->dtype, st_zdir[st], 2 * L.k.nf, &roots);
+                if (rs != FFTB_SUCCESS) return rs;
+            }
+            const long long rows = b->dims[3 * ti] * b->dims[3 * ti + 1];
+            pb.pair = 1;
+            pb.dir = st_zdir[st];
             pb.n = 2 * L.k.nf;
-            pb.lines = (int)(nx * ny);
+            pb.lines = (int)rows;
             pb.scale = st_zdir[st] == 1 && (a.ep_mode & EP_SCALE) ? (float)a.ep_scale : 1.0f;
             pb.roots = (const float2 *)roots;
-            ntiles[p] = (int)(((nx * ny + 1) / 2 + FZ - 1) / FZ);
+            ntiles[p] = (int)(((rows + 1) / 2 + FZ - 1) / FZ);
             smem = std::max(smem, row_group_smem(pb.n));
-        } else if (W > 0) {
-            int rs = prepared(st_ckind[st] * 1000 + L.k.nf,
-                              [&] { return col_group_prepare(b->dtype, st_ckind[st], L.k.nf, &roots); });
-            if (rs != FFTB_SUCCESS) return rs;
-            pb.fast = 1;
-            pb.ckind = st_ckind[st];
-            pb.n = L.k.nf;
-            pb.lines = (int)((st_ckind[st] <= 2 ? ny : nx) * (nz / 2 + 1));
-            pb.ny = (int)ny;
-            pb.nz = (int)nz;
-            pb.scale = (float)a.ep_scale;
-            pb.sign = (float)a.ep_sign;
-            pb.ep_mode = a.ep_mode;
-            pb.roots = (const float2 *)roots;
-            ntiles[p] = (pb.lines + W - 1) / W;
-            smem = std::max(smem, col_group_smem(pb.n));
         }
         binds[p] = pb;
     }
@@ -539,11 +455,8 @@ int build_plan(fftb_batch_s *b, int op, double sign)
         }
     P.nitems = (int)items.size();
     P.smem = smem;
-    // grouped order: within each stage, the items of each line length together; the x and y
-    // stages of lengths that have a column kernel run as one grouped column-kernel launch
-    // each (the fused 3D path's register-resident column FFT, tiles of W lines)
+    // grouped order: within each stage, the items of each line length together
     std::vector<BatchItem> gitems;
-    std::vector<XGroupItem> xitems;
     std::vector<RowGroupItem> ritems;
     gitems.reserve(items.size());
     for (int s = 0; s < P.nstages; ++s) {
@@ -551,7 +464,7 @@ int build_plan(fftb_batch_s *b, int op, double sign)
         for (int i = 0; i < b->count; ++i) nfs.push_back(binds[tpass[i][s]].nf);
         std::sort(nfs.begin(), nfs.end());
         nfs.erase(std::unique(nfs.begin(), nfs.end()), nfs.end());
-        const int ckind = st_ckind[s], zdir = st_zdir[s];
+        const int zdir = st_zdir[s];
         for (int nf : nfs) {
             // nf is the half length for the z stages: the row length is 2 nf
             const int FZ = zdir >= 0 ? row_group_tile_pairs(b->dtype, 2 * nf) : 0;
@@ -561,7 +474,7 @@ int build_plan(fftb_batch_s *b, int op, double sign)
                 const Launch &L0 = P.seq.launches[tpass[0][s]];
                 g.in_buf = L0.in_buf;
                 g.out_buf = L0.out_buf;
-                g.ckind = zdir;
+                g.dir = zdir;
                 int st = row_group_prepare(b->dtype, zdir, 2 * nf, &g.roots);
                 if (st != FFTB_SUCCESS) return st;
                 for (int i = 0; i < b->count; ++i) {
@@ -580,31 +493,6 @@ int build_plan(fftb_batch_s *b, int op, double sign)
                 if (g.count > 0) P.groups.push_back(g);
                 continue;
             }
-            const int W = ckind >= 0 ? col_group_tile_lines(b->dtype, nf) : 0;
-            if (W > 0) {
-                OpPlan::Group g{(int)xitems.size(), 0, nf, 0};
-                g.xcol = true;
-                g.ckind = ckind;
-                const Launch &L0 = P.seq.launches[tpass[0][s]];
-                g.buf = L0.in_buf;
-                g.ep_mode = L0.args.ep_mode;
-                g.ep_scale = L0.args.ep_scale;
-                g.ep_sign = L0.args.ep_sign;
-                int st = col_group_prepare(b->dtype, ckind, nf, &g.roots);
-                if (st != FFTB_SUCCESS) return st;
-                for (int i = 0; i < b->count; ++i) {
-                    const long long nx = b->dims[3 * i], ny = b->dims[3 * i + 1], nz = b->dims[3 * i + 2];
-                    if ((ckind <= 2 ? nx : ny) != nf) continue;
-                    const Launch &L = P.seq.launches[tpass[i][s]];
-                    const long long lines = (ckind <= 2 ? ny : nx) * (nz / 2 + 1);
-                    for (long long t = 0; t < (lines + W - 1) / W; ++t)
-                        xitems.push_back(XGroupItem{(long long)(L.in_off_bytes / complex_bytes(b->dtype)),
-                                                    (int)lines, (int)t, (int)ny, (int)nz});
-                }
-                g.count = (int)xitems.size() - g.offset;
-                if (g.count > 0) P.groups.push_back(g);
-                continue;
-            }
             OpPlan::Group g{(int)gitems.size(), 0, nf, 0};
             for (int i = 0; i < b->count; ++i) {
                 const int p = tpass[i][s];
@@ -612,6 +500,7 @@ int build_plan(fftb_batch_s *b, int op, double sign)
                 g.smem = std::max(g.smem, pass_smem[p]);
                 for (int t = 0; t < ntiles[p]; ++t) gitems.push_back(BatchItem{p, t});
             }
+            g.lkind = binds[gitems[g.offset].pass].lkind;
             g.count = (int)gitems.size() - g.offset;
             if (g.count > 0) P.groups.push_back(g);
         }
@@ -622,9 +511,8 @@ int build_plan(fftb_batch_s *b, int op, double sign)
                      s_binds = al(binds.size() * sizeof(PassBind)), s_deps = al(deps.size() * sizeof(int)),
                      s_nt = al(ntiles.size() * sizeof(int)), s_ctl = al((2 + P.npasses) * sizeof(int));
         const size_t s_gitems = al(gitems.size() * sizeof(BatchItem));
-        const size_t s_xitems = al(xitems.size() * sizeof(XGroupItem));
         const size_t s_ritems = al(ritems.size() * sizeof(RowGroupItem));
-        const size_t tot = s_items + s_args + s_binds + s_deps + s_nt + s_ctl + s_gitems + s_xitems + s_ritems;
+        const size_t tot = s_items + s_args + s_binds + s_deps + s_nt + s_ctl + s_gitems + s_ritems;
         cudaError_t e = cudaMalloc(&P.blob, tot);
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -638,7 +526,6 @@ int build_plan(fftb_batch_s *b, int op, double sign)
         P.d_ntiles = (int *)q; q += s_nt;
         P.d_ctl = (int *)q; q += s_ctl;
         P.d_gitems = (BatchItem *)q; q += s_gitems;
-        P.d_xitems = (XGroupItem *)q; q += s_xitems;
         P.d_ritems = (RowGroupItem *)q;
         e = cudaMemcpy(P.d_items, items.data(), items.size() * sizeof(BatchItem), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemcpy(P.d_passes, args.data(), args.size() * sizeof(PassArgs), cudaMemcpyHostToDevice);
@@ -648,15 +535,13 @@ int build_plan(fftb_batch_s *b, int op, double sign)
         if (e == cudaSuccess) e = cudaMemset(P.d_ctl, 0, (2 + P.npasses) * sizeof(int));
         if (e == cudaSuccess)
             e = cudaMemcpy(P.d_gitems, gitems.data(), gitems.size() * sizeof(BatchItem), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess && !xitems.empty())
-            e = cudaMemcpy(P.d_xitems, xitems.data(), xitems.size() * sizeof(XGroupItem), cudaMemcpyHostToDevice);
         if (e == cudaSuccess && !ritems.empty())
             e = cudaMemcpy(P.d_ritems, ritems.data(), ritems.size() * sizeof(RowGroupItem), cudaMemcpyHostToDevice);
         // the limit is per kernel, not per plan: raise it to the maximum once, so a later
         // plan with a smaller need cannot lower it under an earlier plan's launches
         for (const OpPlan::Group &g : P.groups)
-            if (e == cudaSuccess && !g.xcol && !g.zrow && g.smem > 48 * 1024)
-                e = raise_smem_limit(batch_group_fn(g.nf));
+            if (e == cudaSuccess && !g.zrow && g.smem > 48 * 1024)
+                e = raise_smem_limit(batch_group_fn(g.nf, g.lkind));
         if (e != cudaSuccess) return set_status_from_cuda(e);
         if (smem > 48 * 1024) {
             e = raise_smem_limit((const void *)batch_persistent_kernel);
@@ -691,15 +576,8 @@ int launch_groups(OpPlan &P, const void *in, void *out, void *work, cudaStream_t
     const void *bufs[3] = {in, out, work};
     for (const OpPlan::Group &g : P.groups) {
         if (g.zrow) {
-            int st = launch_row_group(g.ckind, 2 * g.nf, P.d_ritems + g.offset, g.count, bufs[g.in_buf],
+            int st = launch_row_group(g.dir, 2 * g.nf, P.d_ritems + g.offset, g.count, bufs[g.in_buf],
                                       const_cast<void *>(bufs[g.out_buf]), g.roots, s);
-            if (st != FFTB_SUCCESS) return st;
-            continue;
-        }
-        if (g.xcol) {
-            void *data = g.buf == B_IN ? const_cast<void *>(in) : (g.buf == B_OUT ? out : work);
-            int st = launch_col_group(g.ckind, g.nf, P.d_xitems + g.offset, g.count, data, g.roots, g.ep_mode,
-                                      g.ep_scale, g.ep_sign, s);
             if (st != FFTB_SUCCESS) return st;
             continue;
         }
@@ -707,7 +585,7 @@ int launch_groups(OpPlan &P, const void *in, void *out, void *work, cudaStream_t
         const PassArgs *passes = P.d_passes;
         const PassBind *binds = P.d_binds;
         void *args[] = {&items, &passes, &binds, &in, &out, &work};
-        cudaError_t e = cudaLaunchKernel(batch_group_fn(g.nf), dim3((unsigned)g.count), dim3(kBatchThreads), args,
+        cudaError_t e = cudaLaunchKernel(batch_group_fn(g.nf, g.lkind), dim3((unsigned)g.count), dim3(kBatchThreads), args,
                                          g.smem, s);
         if (e != cudaSuccess) return set_status_from_cuda(e);
     }

@@ -1,6 +1,6 @@
-// fftb_coltile.cuh -- the register-resident column tile of the x column kernels and the
-// row-pair tile of the grouped z rows, shared by the fused 3D / 4D kernels and the batch
-// kernels (device templates and the column epilogue parameters).
+// fftb_coltile.cuh -- the register-resident column tile of the x column kernels (fused 3D / 4D) and the
+// row-pair tile of the grouped z rows (batch kernels): device templates and the column epilogue
+// parameters.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -33,8 +33,8 @@ struct XColEp {
 
 template <int NX> struct XColShape {
     static constexpr int T = RegFFTShape<NX>::T;
-    static constexpr int W = 256 / T;      // columns per CTA (48, 96 points: T = 3, 6, and the
-    static constexpr int NT = 256;         // threads past T * W idle)
+    static constexpr int W = 256 / T;      // columns per CTA
+    static constexpr int NT = 256;
 };
 
 // TC: the first radix-16 stage runs on the tensor cores (fftb_tc.cuh, float only)
@@ -44,46 +44,6 @@ __device__ __forceinline__ void xcol_fft(cpx<R> (&v)[16], cpx<R> *scr, const cpx
 {
     using C = cpx<R>;
     constexpr int T = XColShape<NX>::T, W = XColShape<NX>::W;
-    if constexpr (16 % T != 0) {
-        // T = 3 or 6 threads per column (48 or 96 points): thread t runs the second-stage DFTs
-        // of k1 = t, t + T, ... < 16, and one more exchange brings the results back to the
-        // layout v[j] = X[t + T j]; threads past T * W (t = T) take part in the barriers only
-        static_assert(!TC, "tensor-core form: power-of-two columns only");
-        const bool act = t < T;
-        const int tt = act ? t : 0;
-        dft16<SIGN, C, R>(v);
-#pragma unroll
-        for (int k1 = 1; k1 < 16; ++k1) v[k1] = twiddle_mul<SIGN>(v[k1], tw, tt * k1);
-        __syncthreads();
-        if (act) {
-#pragma unroll
-            for (int k1 = 0; k1 < 16; ++k1) scr[(k1 * T + t) * W + col] = v[k1];
-        }
-        __syncthreads();
-        constexpr int A = (16 + T - 1) / T;
-        C res[A][T];
-#pragma unroll
-        for (int a = 0; a < A; ++a) {
-            const int k1 = tt + T * a;
-            const bool valid = act && k1 < 16;
-#pragma unroll
-            for (int q = 0; q < T; ++q) res[a][q] = valid ? scr[(k1 * T + q) * W + col] : mk<R>(R(0), R(0));
-            dft_small<SIGN, T, C, R>(res[a]);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int a = 0; a < A; ++a) {
-            const int k1 = tt + T * a;
-            if (act && k1 < 16) {
-#pragma unroll
-                for (int k2 = 0; k2 < T; ++k2) scr[(k1 + 16 * k2) * W + col] = res[a][k2];
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = act ? scr[(t + T * j) * W + col] : mk<R>(R(0), R(0));
-        return;
-    }
     if constexpr (TC) tc_dft16<SIGN>(v, stage, F, (int)(threadIdx.x & 31));
     else dft16<SIGN, C, R>(v);
 #pragma unroll
@@ -194,8 +154,7 @@ __device__ __forceinline__ void xcol_tile(cpx<R> *data, long long stride, int nc
     const int t = tid / W, col = tid - (tid / W) * W;
     for (int i = tid; i < NX; i += 256) tw[i] = roots[i];
     const int cg0 = tile * W + col;
-    const bool act = t < T;  // false only for the idle threads of 48- and 96-point columns
-    const bool ok = act && cg0 < ncols;
+    const bool ok = cg0 < ncols;
     data += (size_t)batch * bstride;
     C *p = data + (ok ? cg0 : 0);
     C v[16];
@@ -214,7 +173,7 @@ __device__ __forceinline__ void xcol_tile(cpx<R> *data, long long stride, int nc
         for (int r = 0; r < 16; ++r) v[r] = scr[col * RP + t + T * r];
     } else {
 #pragma unroll
-        for (int r = 0; r < 16; ++r) v[r] = act ? p[(size_t)(t + T * r) * stride] : mk<R>(R(0), R(0));
+        for (int r = 0; r < 16; ++r) v[r] = p[(size_t)(t + T * r) * stride];
     }
     __syncthreads();
     if (MODE == 1 || MODE == 4) xcol_fft<R, NX, +1, TC>(v, scr, tw, t, col, stage, F);
@@ -239,42 +198,6 @@ __device__ __forceinline__ void xcol_tile(cpx<R> *data, long long stride, int nc
     } else if (ok) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) p[(size_t)(t + T * j) * stride] = v[j];
-    }
-}
-
-// The y FFT (MODE 0 forward, 1 inverse) of one tile of lines (x, kz) of a 3D spectrum
-// [nx][ny][nzh], kz fastest, W lines per tile, so a warp reads 32 consecutive lines of a y row
-// (contiguous within each x).  it.ncols holds nx * nzh, it.tile the tile, it.ny / it.nz the
-// spectrum's sizes, it.off its offset from data.
-template <int NY, int MODE>
-__device__ __forceinline__ void ycol_tile(const XGroupItem &it, float2 *__restrict__ data,
-                                          const float2 *__restrict__ roots)
-{
-    using C = float2;
-    constexpr int T = XColShape<NY>::T, W = XColShape<NY>::W;
-    constexpr int RP = NY + 1;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C *scr = reinterpret_cast<C *>(smem_raw);
-    C *tw = scr + (16 * T * W > W * RP ? 16 * T * W : W * RP);
-    const int tid = threadIdx.x;
-    const int t = tid / W, col = tid - (tid / W) * W;
-    for (int i = tid; i < NY; i += 256) tw[i] = roots[i];
-    const int nzh = it.nz / 2 + 1;
-    const int l = it.tile * W + col;
-    const bool act = t < T;  // false only for the idle threads of 48- and 96-point lines
-    const bool ok = act && l < it.ncols;
-    const int lc = ok ? l : 0;
-    const int x = lc / nzh, kz = lc - (lc / nzh) * nzh;
-    C *p = data + it.off + (long long)x * it.ny * nzh + kz;
-    C v[16];
-#pragma unroll
-    for (int r = 0; r < 16; ++r) v[r] = act ? p[(size_t)(t + T * r) * nzh] : mk<float>(0.f, 0.f);
-    __syncthreads();
-    TcDft16 F;
-    xcol_fft<float, NY, MODE == 1 ? +1 : -1, false>(v, scr, tw, t, col, nullptr, F);
-    if (ok) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) p[(size_t)(t + T * j) * nzh] = v[j];
     }
 }
 

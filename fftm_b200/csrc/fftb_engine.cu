@@ -276,6 +276,7 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
         Launch S;
         memset(&S.args, 0, sizeof(S.args));
         S.fn = nullptr;
+        S.line = nullptr;
         S.programmatic = 0;
         S.in_buf = p.in_buf;
         S.out_buf = p.out_buf;
@@ -407,12 +408,14 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
     L.smem = smem_of(G);
     long long ncta = (nlines + G - 1) / G;
     L.fn = L.k.fn;
+    L.line = nullptr;
     L.programmatic = line ? 1 : 0;
     if (line) {
         // the thread mapping follows the input side; a side of the other order, or with blocked
         // points, is staged through shared memory
         const LineKernelInfo &k = *r.find_line(dtype, nf, a.in_pts_fast ? 1 : 0);
         if ((p.ep_mode & ~(EP_SCALE | EP_HALFW | EP_TWIDDLE | EP_DERIV)) != 0 && p.kind != K_SANDWICH) return FFTB_ERROR_INVALID_VALUE;
+        L.line = &k;
         a.line_in = !p.in_blk && (!k.row || p.is == 1);
         a.line_out = a.out_pts_fast == a.in_pts_fast && !p.out_blk && (!k.row || p.os == 1);
         line_divisors(a);

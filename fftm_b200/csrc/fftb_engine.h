@@ -54,11 +54,13 @@ struct AxisPass {
 };
 
 struct LongLine;
+struct LineKernelInfo;
 
 struct Launch {
     PassArgs args;
     PassKernelInfo k;    // the pass kernel's tile of this length (the batch kernels run it)
     const void *fn;      // the kernel this launch runs: the line kernel, or the chirp-z pass
+    const LineKernelInfo *line;  // its line kernel (null: chirp-z or a long-line step)
     int programmatic;    // fn waits for its predecessor itself (programmatic launch)
     int in_buf, out_buf;
     size_t in_off_bytes, out_off_bytes;

@@ -600,35 +600,6 @@ __global__ void __launch_bounds__(256, 3) xcol_kernel(cpx<R> *data, long long st
     xcol_tile<R, NX, MODE, TC>(data, stride, ncols, bstride, tdata, roots, ep, (int)blockIdx.x, (int)blockIdx.y);
 }
 
-// One launch over the column tiles of many 3D spectra of one x length (the batched
-// transforms' x stage; MODE 0 forward, 1 inverse, 2 sandwich): item i is tile items[i].tile of
-// the spectrum at data + items[i].off with ny * (nz/2 + 1) columns; the spectral multiply
-// takes that spectrum's ny and nz.
-template <int NX, int MODE>
-__global__ void __launch_bounds__(256, 2) xcol_group_kernel(const XGroupItem *__restrict__ items,
-                                                         float2 *__restrict__ data,
-                                                         const float2 *__restrict__ roots, XColEp ep)
-{
-    const XGroupItem it = items[blockIdx.x];
-    ep.ny = it.ny;
-    ep.nz = it.nz;
-    ep.nzh = it.nz / 2 + 1;
-    ep.hn = it.nz;
-    xcol_tile<float, NX, MODE, false>(data + it.off, it.ncols, it.ncols, 0, nullptr, roots, ep, it.tile, 0);
-}
-
-// The y FFT (MODE 0 forward, 1 inverse) of many 3D spectra [nx][ny][nzh] of one y length in
-// one launch: the lines (x, kz) of a spectrum, kz fastest, in tiles of W lines, so a warp
-// reads 32 consecutive lines of a y row (contiguous within each x); the FFT is the column
-// kernel's register-resident one.  items[i].ncols holds nx * nzh (the lines), .tile the
-// tile, .ny / .nz the spectrum's sizes.
-template <int NY, int MODE>
-__global__ void __launch_bounds__(256, 2) ycol_group_kernel(const XGroupItem *__restrict__ items,
-                                                         float2 *__restrict__ data,
-                                                         const float2 *__restrict__ roots)
-{
-    ycol_tile<NY, MODE>(items[blockIdx.x], data, roots);
-}
 // ------------------------------------------------------------------ x column kernel, TMA ring
 // Persistent form of xcol_kernel (MODE 0, 1, 2) for 16-byte aligned spectra: each CTA walks
 // the tiles (W columns x NX rows; blockIdx.x, + gridDim.x, ...) with NSTAGE tiles in flight,
@@ -1062,41 +1033,6 @@ int launch_xcol(const Fused3D &f, int mode, void *data, const EpValues *ep, cuda
 } // namespace
 
 namespace {
-// kind: 0 x forward, 1 x inverse, 2 x sandwich, 3 y forward, 4 y inverse
-const void *col_group_fn(int kind, int n)
-{
-#define FFTB_COLG(N)                                                                                                   \
-    case N:                                                                                                            \
-        return kind == 0   ? (const void *)&xcol_group_kernel<N, 0>                                                    \
-               : kind == 1 ? (const void *)&xcol_group_kernel<N, 1>                                                    \
-               : kind == 2 ? (const void *)&xcol_group_kernel<N, 2>                                                    \
-               : kind == 3 ? (const void *)&ycol_group_kernel<N, 0>                                                    \
-                           : (const void *)&ycol_group_kernel<N, 1>;
-    if (kind < 0 || kind > 4) return nullptr;
-    switch (n) {
-        FFTB_COLG(32)
-        FFTB_COLG(48)
-        FFTB_COLG(64)
-        FFTB_COLG(96)
-        FFTB_COLG(128)
-        FFTB_COLG(256)
-    default:
-        return nullptr;
-    }
-#undef FFTB_COLG
-}
-
-} // namespace
-
-// dynamic shared memory of a column tile: the exchange / transposing area and the root table
-size_t col_group_smem(int n)
-{
-    const int T = n / 16, W = 256 / T;
-    const size_t scr = (size_t)16 * T * W > (size_t)W * (n + 1) ? (size_t)16 * T * W : (size_t)W * (n + 1);
-    return sizeof(float2) * (scr + (size_t)n);
-}
-
-namespace {
 const void *row_group_fn(int dir, int nz)
 {
     switch (nz) {
@@ -1117,9 +1053,11 @@ size_t row_group_smem(int nz)
     return sizeof(float2) * (size_t)(256 / T) * region;
 }
 
-// Rows of 32 points are left to the pass kernel: two threads per FFT read and write 8 bytes
-// per row at a time, a quarter of a sector, and measured slower than its staged loads
-// (67 / 88 us against 58 / 61 us for the R2C / C2R of the 512-shape batch's 32-point rows).
+// Rows of 64 points and more: two real rows share one complex transform, 65 / 76 us for the R2C / C2R
+// of the 512-shape batch's 64-point rows and 127 / 131 us for its 128-point rows, against 71 / 77
+// and 149 / 156 us for the line kernel's half-length lines.  At 32 points two threads per FFT
+// read and write 8 bytes of a row at a time, a quarter of a sector: 67 / 88 us against the line
+// kernel's 48 / 47.
 int row_group_tile_pairs(int dtype, int nz)
 {
     return dtype == FFTB_F32 && nz >= 64 && row_group_fn(0, nz) ? 256 / (nz / 16) : 0;
@@ -1141,40 +1079,6 @@ int launch_row_group(int dir, int nz, const RowGroupItem *items, int nitems, con
     const float2 *rt = (const float2 *)roots;
     void *args[] = {&items, &in, &out, &rt};
     return set_status_from_cuda(cudaLaunchKernel(fn, dim3((unsigned)nitems), dim3(256), args, row_group_smem(nz), s));
-}
-
-int col_group_tile_lines(int dtype, int n)
-{
-    return dtype == FFTB_F32 && col_group_fn(0, n) ? 256 / (n / 16) : 0;
-}
-
-int col_group_prepare(int dtype, int kind, int n, void **roots)
-{
-    if (dtype != FFTB_F32 || !col_group_fn(kind, n)) return FFTB_ERROR_UNSUPPORTED_SIZE;
-    int st = configure(col_group_fn(kind, n), col_group_smem(n));
-    if (st != FFTB_SUCCESS) return st;
-    return engine_roots(dtype, n, roots);
-}
-
-int launch_col_group(int kind, int n, const XGroupItem *items, int nitems, void *data, const void *roots,
-                     int ep_mode, double scale, double sign, cudaStream_t s)
-{
-    const void *fn = col_group_fn(kind, n);
-    if (!fn || nitems <= 0) return FFTB_ERROR_INVALID_VALUE;
-    const size_t smem = col_group_smem(n);
-    float2 *d = (float2 *)data;
-    const float2 *rt = (const float2 *)roots;
-    if (kind >= 3) {
-        void *args[] = {&items, &d, &rt};
-        return set_status_from_cuda(cudaLaunchKernel(fn, dim3((unsigned)nitems), dim3(256), args, smem, s));
-    }
-    EpValues ev;
-    ev.mode = ep_mode;
-    ev.scale = scale;
-    ev.sign = sign;
-    XColEp x = make_ep(&ev);
-    void *args[] = {&items, &d, &rt, &x};
-    return set_status_from_cuda(cudaLaunchKernel(fn, dim3((unsigned)nitems), dim3(256), args, smem, s));
 }
 
 int fused3d_clusters(int dtype, long long nx, long long ny, long long nz, int *clusters, int cap)

@@ -38,24 +38,6 @@ int fused3d_forward_adjoint(const Fused3D &f, void *gspec, void *greal, cudaStre
 int fused3d_backward_adjoint(const Fused3D &f, const void *greal, void *gspec, cudaStream_t s, LaunchTimer *t);
 int fused3d_num_launches(const Fused3D &f, int which);
 
-// The x or y FFTs of many f32 3D spectra [nx][ny][nz/2+1] of one line length in one launch,
-// one CTA per tile of lines, with the column kernel's register-resident FFT (the batched
-// transforms' column stages).  kind: 0 x forward, 1 x inverse, 2 x sandwich (forward,
-// spectral multiply, inverse), 3 y forward, 4 y inverse.
-struct XGroupItem {
-    long long off;  // complex elements from the buffer base to the spectrum
-    int ncols;      // lines of the spectrum: x kinds ny * (nz/2 + 1), y kinds nx * (nz/2 + 1)
-    int tile;       // tile of col_group_tile_lines(n) lines
-    int ny, nz;
-};
-// 0 when no grouped column kernel exists for this line length, else the lines per tile
-int col_group_tile_lines(int dtype, int n);
-// Raises the kernel's shared-memory limit and returns the root table of length n.
-int col_group_prepare(int dtype, int kind, int n, void **roots);
-// ep_mode / scale / sign: the sandwich's multiply (EP_SCALE, EP_POISSON as the pass epilogue)
-int launch_col_group(int kind, int n, const XGroupItem *items, int nitems, void *data, const void *roots,
-                     int ep_mode, double scale, double sign, cudaStream_t s);
-
 // The z stage of many f32 3D transforms of one z length (32-256, a power of two) in one launch:
 // R2C (dir 0) or scaled C2R (dir 1) of two contiguous real rows per complex FFT.
 struct RowGroupItem {
@@ -66,9 +48,8 @@ struct RowGroupItem {
     float scale;     // C2R output scale
 };
 int row_group_tile_pairs(int dtype, int nz);
-// dynamic shared memory of one row-pair tile / one column tile
+// dynamic shared memory of one row-pair tile
 size_t row_group_smem(int nz);
-size_t col_group_smem(int n);
 int row_group_prepare(int dtype, int dir, int nz, void **roots);
 int launch_row_group(int dir, int nz, const RowGroupItem *items, int nitems, const void *in, void *out,
                      const void *roots, cudaStream_t s);

@@ -211,7 +211,7 @@ template <typename R, int N, bool ROW> struct LineShape {
     }
     static constexpr int col_lines()
     {
-        const int lo = sizeof(R) == 4 ? 8 : 4, hi = sizeof(R) == 4 ? 64 : 32;
+        const int lo = sizeof(R) == 4 ? 8 : 4, hi = sizeof(R) == 4 ? 128 : 32;
         int g = 1;
         while (g * 2 * T <= 256 && g < hi) g *= 2;
         while (g < lo && g * 2 * T <= 1024) g *= 2;
@@ -496,9 +496,12 @@ template <bool U, bool B> struct LineDir {
     static constexpr bool unit = U, back = B;
 };
 
-template <typename R, int N, bool ROW, bool SAND>
-__global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>::MINB)
-    fftb_line_kernel(const __grid_constant__ PassArgs a)
+// One CTA's lines: tile `tile` of the pass.  BATCH: called from the batch kernels, whose blocks may
+// have more threads than the tile (the extra ones repeat the first and store nothing) and whose
+// passes have no staged side, no long-line twiddle and no programmatic launch.
+template <typename R, int N, bool ROW, bool SAND, bool BATCH>
+__device__ __forceinline__ void line_body(const PassArgs &__restrict__ a, const void *in_ptr, void *out_ptr,
+                                          long long tile, unsigned char *smem_raw, long long *soff)
 {
     using C = cpx<R>;
     using S = LineShape<R, N, ROW>;
@@ -508,16 +511,17 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
     // the last stage's radix (the sandwich ends with the reversed plan's last, r_0)
     constexpr int RL = SAND ? P.r[0] : P.r[P.S - 1], NBL = N / RL, PERL = (NBL + T - 1) / T;
     constexpr int PH = (N / 2 + T) / T;  // pairs (k, N - k), k = t + T i <= N/2, of a thread
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ long long soff[G];  // line offsets of a staged side
+    // an extra thread repeats another's exchange writes, which only block-wide barriers order
+    static_assert(!BATCH || !S::WARP || NT == 256, "whole tiles where a warp orders its own exchanges");
     C *s = reinterpret_cast<C *>(smem_raw);
-    const int tid = threadIdx.x;
+    const int tid = BATCH && threadIdx.x >= NT ? threadIdx.x - NT : threadIdx.x;
     const int g = ROW ? tid / T : tid % G, t = ROW ? tid - g * T : tid / G;
     C *ln = ROW ? s + g * S::LP : s + g;
     C *st = s + g * S::SP;  // this line in a staged side
     // threads past the last line repeat it and store nothing
-    const bool act = (long long)blockIdx.x * G + g < a.nlines;
-    const long long l = act ? (long long)blockIdx.x * G + g : a.nlines - 1;
+    const bool has = tile * G + g < a.nlines;
+    const bool act = has && (!BATCH || threadIdx.x < NT);
+    const long long l = has ? tile * G + g : a.nlines - 1;
     int b0, b1, b2;
     if (a.c_shift >= 0) {  // l < 2^31: the divisions as multiplications (PassArgs)
         const unsigned q = (unsigned)(((unsigned long long)(unsigned)l * a.c0_mul) >> (a.c_shift & 63));
@@ -537,13 +541,13 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
     // it is an ordinary load (the tables alone are read as constants).  Back to back: 192^3 f32
     // Poisson 76.9 -> 66.4 us, 32^3 f64 25.4 -> 18.2, 2048^2 forward 26.7 -> 21.8, 256^3 f64 round
     // trip 306 -> 302.
-    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;\n" ::: "memory");
+    if constexpr (!BATCH) asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;\n" ::: "memory");
     const int kind = SAND ? (int)K_SANDWICH : a.kind;
     const bool half = !SAND && a.half;
     // the direct side of a ROW pass has unit stride
     const long long is = ROW ? 1 : a.is, os = ROW ? 1 : a.os;
-    const bool in_t = !a.line_in, out_t = !a.line_out;
-    const long long left = a.nlines - (long long)blockIdx.x * G;
+    const bool in_t = !BATCH && !a.line_in, out_t = !BATCH && !a.line_out;
+    const long long left = a.nlines - tile * G;
     const int rows = left < G ? (int)left : G;  // lines of this CTA
 
     C v[S::E];
@@ -627,7 +631,7 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
         staged(kind == K_C2R ? (half ? N + 1 : N / 2 + 1) : N, a.in_pts_fast, [&](int gg, int p) {
             C *d = &s[gg * S::SP + p];
             if (kind == K_R2C) {
-                const R *src = reinterpret_cast<const R *>(a.in) + soff[gg];
+                const R *src = reinterpret_cast<const R *>(in_ptr) + soff[gg];
                 if (half) {
                     cp_async<sizeof(R)>(&d->x, src + (2 * p) * a.is, true);
                     cp_async<sizeof(R)>(&d->y, src + (2 * p + 1) * a.is, true);
@@ -638,7 +642,7 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
             } else {
                 const long long pi =
                     a.in_blk ? (long long)(p / a.in_blk) * a.in_hi + (long long)(p % a.in_blk) * a.is : p * a.is;
-                cp_async<sizeof(C)>(d, reinterpret_cast<const C *>(a.in) + soff[gg] + pi, true);
+                cp_async<sizeof(C)>(d, reinterpret_cast<const C *>(in_ptr) + soff[gg] + pi, true);
             }
         });
         cp_async_wait_all();
@@ -651,12 +655,12 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
             __syncthreads();  // the staged lines are read before the exchanges overwrite them
         }
     } else if (!SAND && kind == K_R2C) {
-        const R *in = reinterpret_cast<const R *>(a.in) + io;
+        const R *in = reinterpret_cast<const R *>(in_ptr) + io;
         if (half && a.pair_io) load(2, [&](int, long long o) { return *reinterpret_cast<const C *>(in + o); });
         else if (half) load(2 * is, [&](int, long long o) { return mk<R>(in[o], in[o + is]); });
         else load(is, [&](int, long long o) { return mk<R>(in[o], R(0)); });
     } else {
-        const C *in = reinterpret_cast<const C *>(a.in) + io;
+        const C *in = reinterpret_cast<const C *>(in_ptr) + io;
         if (SAND || kind != K_C2R) load(is, [&](int, long long o) { return in[o]; });
         else if (half) load_packed(false, in, is);
         else load(is, [&](int p, long long) { return extend(p, in[(p <= N / 2 ? p : N - p) * is]); });
@@ -699,7 +703,7 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
     // ------------------------------------------------------------ epilogue
     const bool inv = SAND || kind == K_C2C_INV || kind == K_C2R;  // result i is point -i mod N
     if (!SAND && a.ep_mode) {
-        if (a.ep_mode & EP_TWIDDLE) {
+        if (!BATCH && (a.ep_mode & EP_TWIDDLE)) {
             // the four-step twiddle of a long line: p < L1 and j < L2, so p j < L needs no reduction
             const C *eptw = reinterpret_cast<const C *>(a.ep_tw);
             const int j = a.ep_src[0] == 1 ? b0 : (a.ep_src[0] == 2 ? b1 : b2);
@@ -780,7 +784,7 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
                 }
             }
         } else if (act) {
-            C *pa = reinterpret_cast<C *>(a.out) + oo + t * os, *pb = reinterpret_cast<C *>(a.out) + oo + (N - t) * os;
+            C *pa = reinterpret_cast<C *>(out_ptr) + oo + t * os, *pb = reinterpret_cast<C *>(out_ptr) + oo + (N - t) * os;
 #pragma unroll
             for (int i = 0; i < PH; ++i, pa += T * os, pb -= T * os) {
                 if (i + 1 < PH || t + T * i <= N / 2) {
@@ -794,7 +798,7 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
         store(1, [&](int p, long long, C z) { st[p] = z; });
     } else if (act) {
         if (!SAND && kind == K_C2R) {
-            R *o = reinterpret_cast<R *>(a.out) + oo;
+            R *o = reinterpret_cast<R *>(out_ptr) + oo;
             if (!half) store(os, [&](int, long long f, C z) { o[f] = z.x; });
             else if (a.pair_io) store(2, [&](int, long long f, C z) { *reinterpret_cast<C *>(o + f) = z; });
             else
@@ -803,7 +807,7 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
                     o[f + os] = z.y;
                 });
         } else {
-            C *o = reinterpret_cast<C *>(a.out) + oo;
+            C *o = reinterpret_cast<C *>(out_ptr) + oo;
             if (!SAND && kind == K_R2C) store(os, [&](int p, long long f, C z) { if (p <= N / 2) o[f] = z; });
             else store(os, [&](int, long long f, C z) { o[f] = z; });
         }
@@ -815,7 +819,7 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
         staged(kind == K_R2C ? (half ? N + 1 : N / 2 + 1) : N, a.out_pts_fast, [&](int gg, int p) {
             const C z = s[gg * S::SP + p];
             if (kind == K_C2R) {
-                R *o = reinterpret_cast<R *>(a.out) + soff[gg];
+                R *o = reinterpret_cast<R *>(out_ptr) + soff[gg];
                 if (half) {
                     o[(2 * p) * a.os] = z.x;
                     o[(2 * p + 1) * a.os] = z.y;
@@ -823,7 +827,7 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
                     o[p * a.os] = z.x;
                 }
             } else {
-                C *o = reinterpret_cast<C *>(a.out) + soff[gg];
+                C *o = reinterpret_cast<C *>(out_ptr) + soff[gg];
                 if (a.out_blk) {  // a slab exchange's pack: block q of the points, or a peer's buffer
                     const int q = p / a.out_blk;
                     C *base = a.out_peer[q] ? reinterpret_cast<C *>(a.out_peer[q]) + soff[gg] : o + (long long)q * a.out_hi;
@@ -834,6 +838,15 @@ __global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>
             }
         });
     }
+}
+
+template <typename R, int N, bool ROW, bool SAND>
+__global__ void __launch_bounds__(LineShape<R, N, ROW>::NT, LineShape<R, N, ROW>::MINB)
+    fftb_line_kernel(const __grid_constant__ PassArgs a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ long long soff[LineShape<R, N, ROW>::G];  // line offsets of a staged side
+    line_body<R, N, ROW, SAND, false>(a, a.in, a.out, blockIdx.x, smem_raw, soff);
 }
 
 // what the host needs of one line length and mapping

@@ -263,8 +263,9 @@ int fftb_batch_layout(fftb_batch batch, long long *real_offsets, long long *spec
 int fftb_batch_work_size(fftb_batch batch, size_t *bytes);
 int fftb_batch_set_work_area(fftb_batch batch, void *work);
 int fftb_batch_set_stream(fftb_batch batch, void *stream);
-/* Tuning knobs chosen by the autotuner: tiles of (default lines)/tiles_scale lines and
- * at most ctas_per_sm persistent CTAs per SM (0: the occupancy limit). */
+/* Tuning knobs chosen by the autotuner: tiles_scale (kept in the configs; the tiles have one
+ * size each, so every value runs the same) and at most ctas_per_sm persistent CTAs per SM (0: the
+ * occupancy limit). */
 int fftb_batch_set_tuning(fftb_batch batch, int tiles_scale, int ctas_per_sm);
 /* op: FFTB_BATCH_*; sign: Poisson sign (ignored otherwise); mode: 0 sequential plain
  * launches, 1 one persistent launch, 2 persistent launch replayed from a CUDA graph,
