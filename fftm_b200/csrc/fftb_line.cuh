@@ -13,7 +13,8 @@
 //
 // Lines are n = r_0 r_1 ... points (Stockham order: Govindaraju et al., "High performance
 // discrete Fourier transforms on graphics processors", SC 2008); the plan takes the fewest
-// stages of radices up to 16 and, of those, the most even ones, so a stage's n / r_i butterflies
+// stages of radices up to 16 (float lines above 256 points: two of up to 32, line_plan) and, of those,
+// the most even ones, so a stage's n / r_i butterflies
 // fill the line's T threads.
 //
 // Two thread mappings: ROW (the points of a line are neighbours in memory: consecutive threads
@@ -40,10 +41,13 @@ struct LinePlan {
     int E = 1;                 // complex values a thread holds
 };
 
-__host__ __device__ constexpr bool line_radix_ok(int r) { return r >= 2 && r <= 16; }
+__host__ __device__ constexpr bool line_radix_ok(int r)
+{
+    return (r >= 2 && r <= 16) || r == 18 || r == 20 || r == 24 || r == 25 || r == 30 || r == 32;
+}
 
 // The most even factorisation of n into S radices (descending): minimal largest radix, then
-// maximal smallest.  false if there is none.
+// maximal smallest, none above top.  false if there is none.
 __host__ __device__ constexpr bool line_factor(int n, int S, int top, int *out)
 {
     if (S == 1) {
@@ -53,8 +57,8 @@ __host__ __device__ constexpr bool line_factor(int n, int S, int top, int *out)
     }
     int best[5] = {};
     bool have = false;
-    for (int r = top < 16 ? top : 16; r >= 2; --r) {
-        if (n % r) continue;
+    for (int r = top; r >= 2; --r) {
+        if (n % r || !line_radix_ok(r)) continue;
         int rest[5] = {};
         if (!line_factor(n / r, S - 1, r, rest)) continue;
         // largest radix r falls with the loop, so the last hit has the smallest largest radix;
@@ -72,8 +76,13 @@ __host__ __device__ constexpr bool line_factor(int n, int S, int top, int *out)
 //
 // ROW lines split every composite length (a thread per line would read its points one line
 // apart) and take the larger of equally good thread counts; COL lines the smaller.
-// emax bounds the values a thread holds.
-__host__ __device__ constexpr LinePlan line_plan(int n, bool row, int emax)
+// emax bounds the values a thread holds.  top: the largest radix of a two-stage plan above 256 points.
+// In float up to 32 (64 registers of values, 16 warps per SM): a third stage costs another
+// exchange and set of twiddles, and these kernels are bound by issue and shared-memory
+// wavefronts: 512-point columns of 512^3 241 -> 218 us and their sandwich 369 -> 316 (16 x 32 for
+// 8 x 8 x 8), 400-point columns 311 -> 247 (20 x 20), 480-point sandwich 303 -> 246, 320-point rows
+// 168 -> 138.  In double 32 values would take 128 registers: three stages.
+__host__ __device__ constexpr LinePlan line_plan(int n, bool row, int emax, int top)
 {
     LinePlan p;
     if (n <= 1) return p;
@@ -86,7 +95,7 @@ __host__ __device__ constexpr LinePlan line_plan(int n, bool row, int emax)
             if (!prime) continue;
         }
         int r[5] = {};
-        if (line_factor(n, S, 16, r)) {
+        if (line_factor(n, S, S == 2 && n > 256 ? top : 16, r)) {
             have = true;
             p.S = S;
             for (int i = 0; i < S; ++i) p.r[i] = r[i];
@@ -184,10 +193,10 @@ __host__ __device__ constexpr int line_conflicts(const LinePlan &p, int n, int T
     return c;
 }
 
-constexpr int kLineEmax = 16;  // 16 complex values: 32 (float) or 64 (double) registers
+constexpr int kLineEmax = 16;  // 16 complex values: 32 (float) or 64 (double) registers (radices above take more)
 
 template <typename R, int N, bool ROW> struct LineShape {
-    static constexpr LinePlan P = line_plan(N, ROW, kLineEmax);
+    static constexpr LinePlan P = line_plan(N, ROW, kLineEmax, sizeof(R) == 4 ? 32 : 16);
     static constexpr LinePlan Q = line_reverse(P);
     static constexpr int T = P.T, E = P.E;
     // lines per CTA.  ROW: as near to 256 threads as fills its warps best.  COL: segments of at
@@ -246,13 +255,39 @@ template <typename R, int N, bool ROW> struct LineShape {
     static constexpr size_t EX = (size_t)G * LP;      // exchange area, entries
     static constexpr int SP = (N + 1) | 1;                              // staged line pitch (in_t / out_t)
     static constexpr size_t ST = (size_t)G * SP;
-    // CTAs per SM the registers are budgeted for: 64 registers a thread (float), 128 (double)
-    static constexpr int MINB = (65536 / (sizeof(R) == 4 ? 64 : 128)) / (NT < 32 ? 32 : NT) > 0
-                                    ? (65536 / (sizeof(R) == 4 ? 64 : 128)) / (NT < 32 ? 32 : NT)
+    // CTAs per SM the registers are budgeted for: 64 registers a thread (float; 80 and 128 with
+    // more than 16 and 20 values), 128 (double)
+    static constexpr int MINB = (65536 / (sizeof(R) == 4 ? (E > 20 ? 128 : E > 16 ? 80 : 64) : 128)) / (NT < 32 ? 32 : NT) > 0
+                                    ? (65536 / (sizeof(R) == 4 ? (E > 20 ? 128 : E > 16 ? 80 : 64) : 128)) / (NT < 32 ? 32 : NT)
                                     : 1;
 };
 
 // ---------------------------------------------------------------- butterflies
+// sine and cosine by their power series (|x| <= pi; the terms fall below 1e-40 by the 30th)
+__host__ __device__ constexpr double ct_sin(double x)
+{
+    double t = x, r = x;
+    for (int i = 1; i < 30; ++i) { t *= -x * x / ((2 * i) * (2 * i + 1)); r += t; }
+    return r;
+}
+__host__ __device__ constexpr double ct_cos(double x)
+{
+    double t = 1, r = 1;
+    for (int i = 1; i < 30; ++i) { t *= -x * x / ((2 * i - 1) * (2 * i)); r += t; }
+    return r;
+}
+// exp(2 pi i m / M), m < M
+template <int M> struct CtTable {
+    double c[M] = {}, s[M] = {};
+    constexpr CtTable()
+    {
+        for (int m = 0; m < M; ++m) {
+            const double x = 6.283185307179586476925286766559 * (2 * m > M ? m - M : m) / M;
+            c[m] = ct_cos(x);
+            s[m] = ct_sin(x);
+        }
+    }
+};
 // n = A B with coprime A and B (Good 1958, Thomas 1963: the prime factor algorithm): input
 // index B n1 + A n2, output index k with k = k1 mod A and k = k2 mod B, and no twiddles between.
 __host__ __device__ constexpr int pfa_out(int A, int B, int k1, int k2)
@@ -362,9 +397,39 @@ template <typename R, typename C> __device__ __forceinline__ void dft9(C *v)
 }
 
 // forward DFT of RAD values in registers
+// A x B with the twiddles w_AB^(n k) between
+template <typename R, int A, int B, typename C> __device__ __forceinline__ void dft_ct(C *v)
+{
+    C u[A][B];
+#pragma unroll
+    for (int n = 0; n < B; ++n) {
+        C c[A];
+#pragma unroll
+        for (int m = 0; m < A; ++m) c[m] = v[n + B * m];
+        line_dft<R, A>(c);
+#pragma unroll
+        for (int k = 0; k < A; ++k) {
+            constexpr CtTable<A * B> w{};
+            u[k][n] = n * k == 0 ? c[k] : cmulc(c[k], mk<R>(R(w.c[n * k]), R(w.s[n * k])));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < A; ++k) {
+        line_dft<R, B>(u[k]);
+#pragma unroll
+        for (int m = 0; m < B; ++m) v[k + A * m] = u[k][m];
+    }
+}
+
 template <typename R, int RAD, typename C> __device__ __forceinline__ void line_dft(C *v)
 {
-    if constexpr (RAD == 6) dft_pfa<R, 2, 3>(v);
+    if constexpr (RAD == 18) dft_pfa<R, 2, 9>(v);
+    else if constexpr (RAD == 20) dft_pfa<R, 4, 5>(v);
+    else if constexpr (RAD == 24) dft_pfa<R, 3, 8>(v);
+    else if constexpr (RAD == 30) dft_pfa<R, 2, 15>(v);
+    else if constexpr (RAD == 25) dft_ct<R, 5, 5>(v);
+    else if constexpr (RAD == 32) dft_ct<R, 4, 8>(v);
+    else if constexpr (RAD == 6) dft_pfa<R, 2, 3>(v);
     else if constexpr (RAD == 9) dft9<R>(v);
     else if constexpr (RAD == 10) dft_pfa<R, 2, 5>(v);
     else if constexpr (RAD == 11 || RAD == 13) dft_prime<R, RAD>(v);

@@ -13,7 +13,8 @@ TOL = {"float32": 2e-6, "float64": 4e-15}
 
 # one length per radix, per pair of stages, and the three- to five-stage plans up to the largest
 LENGTHS = [1, 2, 3, 5, 7, 9, 10, 11, 12, 13, 14, 15, 16, 18, 25, 44, 49, 64, 98, 125, 150, 180,
-           192, 208, 225, 243, 250, 256, 343, 500, 512, 675, 1000, 1024, 1250, 2187, 2401, 3125, 4096]
+           192, 208, 225, 243, 250, 256, 288, 300, 320, 343, 360, 384, 400, 432,
+           480, 500, 512, 600, 625, 640, 768, 900, 960, 675, 1000, 1024, 1250, 2187, 2401, 3125, 4096]
 # (points adjacent in memory, lines adjacent) of the input and of the output
 SIDES = [("row", "row"), ("col", "col"), ("row", "col"), ("col", "row")]
 
@@ -89,7 +90,7 @@ def test_line_kinds(F, torch_cuda, n, sides, dtype):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "float64"])
-@pytest.mark.parametrize("shape", [(16, 9, 10), (45, 26, 18), (180, 4, 6), (512, 3, 2), (9, 1000, 4)])
+@pytest.mark.parametrize("shape", [(16, 9, 10), (45, 26, 18), (180, 4, 6), (512, 3, 2), (384, 4, 2), (500, 2, 4), (9, 1000, 4)])
 def test_sandwich(F, torch_cuda, shape, dtype):
     """The x sandwich of the staged solve at one to three stages (the second transform runs the
     radices in reverse), and the row mapping's sandwich in the 4D pencil order."""
