@@ -371,7 +371,6 @@ def main():
     torch.cuda.synchronize()
 
     launches_per_step = ff.num_launches("poisson")
-    ff.timing_enable(launches_per_step * args.steps + 8)
     starts = [torch.cuda.Event(enable_timing=True) for _ in range(args.steps)]
     ends = [torch.cuda.Event(enable_timing=True) for _ in range(args.steps)]
     clocks = ClockSampler(local)
@@ -392,6 +391,13 @@ def main():
     clk = clocks.stop()
     step_ms = [s.elapsed_time(e) for s, e in zip(starts, ends)]
     total_ms = sum(step_ms)
+    # per-launch times in a loop of their own: the events between the launches would keep each from
+    # starting under its predecessor's tail in the timed steps
+    ff.timing_enable(launches_per_step * args.steps + 8)
+    for _ in range(args.steps):
+        flush.zero_()
+        step()
+    torch.cuda.synchronize()
     per_launch = ff.timing_read()
     ff.timing_enable(0)
     total_ms = replicas.max_over_ranks(dist, total_ms, dev)
