@@ -488,21 +488,4 @@ __device__ __forceinline__ void fft_line(cpx<R> *s, const cpx<R> *tw, int NT, in
     stockham_from<R, NF, SIGN, 0, threads_per_line(NF)>(s, tw, NT, t, act);
 }
 
-// Global -> shared staging of BYTES (4, 8 or 16) bytes.  CG = false: asynchronous
-// cp.async (completed by cp_async_wait_all); CG = true: a synchronous load that
-// bypasses L1 (ld.global.cg), for data other CTAs of the same launch wrote.
-template <bool CG, int BYTES> __device__ __forceinline__ void stage_load(void *d, const void *s, bool ok)
-{
-    if constexpr (!CG) {
-        cp_async<BYTES>(d, s, ok);
-    } else if constexpr (BYTES == 4) {
-        *reinterpret_cast<float *>(d) = ok ? __ldcg(reinterpret_cast<const float *>(s)) : 0.f;
-    } else if constexpr (BYTES == 8) {
-        *reinterpret_cast<float2 *>(d) = ok ? __ldcg(reinterpret_cast<const float2 *>(s)) : make_float2(0.f, 0.f);
-    } else {
-        *reinterpret_cast<float4 *>(d) =
-            ok ? __ldcg(reinterpret_cast<const float4 *>(s)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-}
-
 } // namespace fftb
