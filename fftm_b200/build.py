@@ -22,11 +22,20 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libfftb_b200.so")
 NPARTS = 8        # objects of the pass kernel's instantiations
-LINE_NPARTS = 16  # objects per precision of the line kernel's
+LINE_NPARTS = 64  # objects per precision of the line kernel's
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xfatbin=--compress-mode=size", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
+NVCC_FLAGS = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
               "--expt-relaxed-constexpr", f"-DFFTB_NPARTS={NPARTS}", f"-DFFTB_LINE_NPARTS={LINE_NPARTS}"]
+# An object's device code is one module, which the runtime unpacks and loads whole when the first of
+# its kernels is asked for: the first call of a process on a length pays for that.  The line
+# kernels' (1200 of them) are therefore kept small: 64 objects per precision, about five lengths each,
+# and without -lineinfo, whose records of the inlined stages are 70% of a module (21.3 against
+# 6.0 MB for a sixteenth of the lengths).  Loading one module on a B200: 30 ms in 16 objects with line
+# records, 8.5 ms in 64 with them, 2.4 ms in 64 without; the first 192^3 gradient of a process (two
+# modules and its allocations): 58 ms in 16 objects with records, 6.1 so.
+LINE_FLAGS = ["-Xfatbin=--compress-mode=size"]
+OTHER_FLAGS = ["-lineinfo"]
 
 
 def nvcc() -> str:
@@ -81,15 +90,16 @@ def _jobs():
         src = os.path.join(CSRC, f)
         if f == "fftb_pass_inst.cu":
             for k in range(NPARTS):
-                jobs.append((src, os.path.join(BUILD, f"pass_float_{k}.o"), ["-DFFTB_REAL=float", f"-DFFTB_PART={k}"]))
+                jobs.append((src, os.path.join(BUILD, f"pass_float_{k}.o"),
+                             OTHER_FLAGS + ["-DFFTB_REAL=float", f"-DFFTB_PART={k}"]))
         elif f == "fftb_line_inst.cu":
             for real in ("float", "double"):
                 for k in range(LINE_NPARTS):
                     obj = os.path.join(BUILD, f"line_{real}_{k}.o")
-                    jobs.append((src, obj, [f"-DFFTB_REAL={real}", f"-DFFTB_PART={k}"]))
+                    jobs.append((src, obj, LINE_FLAGS + [f"-DFFTB_REAL={real}", f"-DFFTB_PART={k}"]))
         else:
-            jobs.append((src, os.path.join(BUILD, f[:-3] + ".o"), []))
-    jobs.append((_digest_source(source_digest()), os.path.join(BUILD, "fftb_digest.o"), []))
+            jobs.append((src, os.path.join(BUILD, f[:-3] + ".o"), OTHER_FLAGS))
+    jobs.append((_digest_source(source_digest()), os.path.join(BUILD, "fftb_digest.o"), OTHER_FLAGS))
     return jobs
 
 

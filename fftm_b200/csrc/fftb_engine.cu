@@ -21,9 +21,13 @@
     extern "C" int fftb_line_table_float_part##k(fftb::LineKernelInfo *, int);                                        \
     extern "C" int fftb_line_table_double_part##k(fftb::LineKernelInfo *, int);
 #define FFTB_PARTS8(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7)
-#define FFTB_PARTS16(X) FFTB_PARTS8(X) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15)
+#define FFTB_PARTS64(X)                                                                                               \
+    FFTB_PARTS8(X) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(17) X(18) X(19) X(20) X(21) X(22) X(23)      \
+    X(24) X(25) X(26) X(27) X(28) X(29) X(30) X(31) X(32) X(33) X(34) X(35) X(36) X(37) X(38) X(39) X(40) X(41)       \
+    X(42) X(43) X(44) X(45) X(46) X(47) X(48) X(49) X(50) X(51) X(52) X(53) X(54) X(55) X(56) X(57) X(58) X(59)       \
+    X(60) X(61) X(62) X(63)
 FFTB_PARTS8(FFTB_DECL_PASS)
-FFTB_PARTS16(FFTB_DECL_LINE)
+FFTB_PARTS64(FFTB_DECL_LINE)
 
 namespace fftb {
 
@@ -45,7 +49,7 @@ struct Registry {
 #define FFTB_FN_LINE32(k) fftb_line_table_float_part##k,
 #define FFTB_FN_LINE64(k) fftb_line_table_double_part##k,
         int (*const fp[])(PassKernelInfo *, int) = {FFTB_PARTS8(FFTB_FN_PASS)};
-        int (*const fl[2][16])(LineKernelInfo *, int) = {{FFTB_PARTS16(FFTB_FN_LINE32)}, {FFTB_PARTS16(FFTB_FN_LINE64)}};
+        int (*const fl[2][64])(LineKernelInfo *, int) = {{FFTB_PARTS64(FFTB_FN_LINE32)}, {FFTB_PARTS64(FFTB_FN_LINE64)}};
         PassKernelInfo pb[256];
         for (auto f : fp) {
             const int n = f(pb, 256);
