@@ -18,6 +18,7 @@ Error behaviour follows the reference: API misuse raises :class:`LogicError`
 from __future__ import annotations
 
 import ctypes
+import threading
 
 from . import _lib
 
@@ -92,6 +93,23 @@ def _stream_ptr(stream=None) -> int:
     return _current_raw_stream()
 
 
+class _StreamBinding:
+    """The stream a handle is bound to.  The handle is set only when the stream differs; setting it
+    and noting it are one step under a lock, so that threads which use one object on different
+    streams never leave a note that the handle does not have."""
+
+    def __init__(self):
+        self._bound = 0  # a new handle runs on the null stream
+        self._lock = threading.Lock()
+
+    def bind(self, setter, handle, stream):
+        s = _stream_ptr(stream)
+        if s != self._bound:
+            with self._lock:
+                _check(setter(handle, s), "set_stream")
+                self._bound = s
+
+
 def version() -> str:
     return _lib.load().fftb_version().decode()
 
@@ -126,7 +144,7 @@ class Plan:
                                 batch, ctypes.byref(h), ctypes.byref(ws))
         _check(st, "fftb_plan_create")
         self._h = h
-        self._stream = 0  # the stream the handle is bound to
+        self._stream = _StreamBinding()
         self.work_size = ws.value
 
     def __del__(self):
@@ -139,10 +157,7 @@ class Plan:
         self._h = None
 
     def set_stream(self, stream=None):
-        s = _stream_ptr(stream)
-        if s != self._stream:  # the handle keeps its stream between calls
-            _check(_lib.load().fftb_plan_set_stream(self._h, s), "set_stream")
-            self._stream = s
+        self._stream.bind(_lib.load().fftb_plan_set_stream, self._h, stream)
 
     def set_work_area(self, tensor_or_ptr):
         ptr = tensor_or_ptr if isinstance(tensor_or_ptr, int) else _ptr(tensor_or_ptr)
@@ -318,7 +333,7 @@ class ffts:
         self.dtype = _dtype_code(dtype)
         self.strategy_4d = _STRATEGY[strategy_4d]
         self._h = None
-        self._stream = 0  # the stream the handle is bound to
+        self._stream = _StreamBinding()
         self._dims = None
         self._work = None
 
@@ -388,10 +403,7 @@ class ffts:
         _check(_lib.load().fftb_ffts_set_work_area(self._h, _ptr(tensor)), "set_work_area")
 
     def _bind(self, stream):
-        s = _stream_ptr(stream)
-        if s != self._stream:  # the handle keeps its stream between calls
-            _check(_lib.load().fftb_ffts_set_stream(self._h, s), "set_stream")
-            self._stream = s
+        self._stream.bind(_lib.load().fftb_ffts_set_stream, self._h, stream)
 
     def forward(self, real_in, complex_out, stream=None):
         self._ensure(real_in.dim() if real_in.dim() in (2, 3, 4) else None)
