@@ -201,7 +201,11 @@ template <typename R, int N, bool ROW> struct LineShape {
     static constexpr int T = P.T, E = P.E;
     // lines per CTA.  ROW: as near to 256 threads as fills its warps best.  COL: segments of at
     // least 64 bytes (8 float, 4 double lines) and 256 threads, up to 1024 threads and 160 KB of
-    // exchange area (512^3 f32 Poisson back to back: 1113 us with 64-byte segments, 1137 with 128)
+    // exchange area (512^3 f32 Poisson back to back: 1113 us with 64-byte segments, 1137 with 128).
+    // Double lines of one thread: past 32 lines while the tile is below 6 KB, because a CTA of one warp
+    // with a few values a thread is bound by CTA starts (2^22 points as C2C columns of 1, 2 and 4
+    // points 136 -> 36, 69 -> 25 and 35 -> 22 us, R2C of 4, 8 and 16 points 35 -> 13, 18 -> 11 and
+    // 11 -> 10; longer lines gain nothing, and lose 4% with a staged side).
     static constexpr int row_lines()
     {
         int best = 1, bw = 1 << 30;
@@ -222,7 +226,7 @@ template <typename R, int N, bool ROW> struct LineShape {
     {
         const int lo = sizeof(R) == 4 ? 8 : 4, hi = sizeof(R) == 4 ? 128 : 32;
         int g = 1;
-        while (g * 2 * T <= 256 && g < hi) g *= 2;
+        while (g * 2 * T <= 256 && (g < hi || (g < 128 && g * N < 384))) g *= 2;
         while (g < lo && g * 2 * T <= 1024) g *= 2;
         while (g > 1 && (size_t)g * N * 2 * sizeof(R) > 160 * 1024) g /= 2;
         return g;
