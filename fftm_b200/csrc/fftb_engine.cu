@@ -236,6 +236,23 @@ void line_divisors(PassArgs &a)
     a.c_shift = s0 | (s1 << 6);
 }
 
+// Whether a pass from rows to columns runs the column mapping with its input staged, instead of the
+// row mapping k with its output staged.  Double lines that the row mapping splits do while they are
+// short: a thread of a column tile holds most of a line, where the row tile exchanges and often needs
+// the whole block's barriers for it (2^22 points as C2C of 4, 8 and 35 points 32 -> 26, 31 -> 25 and
+// 51 -> 43 us, R2C of 8 and 16 points 20 -> 15 and 19 -> 14, C2R of 35 points 43 -> 30).  Lines of one
+// stage, odd R2C lines, C2C from 64 and real lines from 48 complex points on are as fast or
+// faster as rows (C2C of 2 points 27 us against 29, R2C of 25 points 23 against 25, of 112 points 15.5
+// against 17.4).  So do the longest C2R lines in float, of which a row tile holds two or one, so
+// that its column segments are 8 bytes (3840 points 29 -> 20 us, 8192 points 42 -> 21; 3456
+// points and below are faster as rows).
+bool columns_from_rows(int dtype, int kind, bool half, const LineKernelInfo &k)
+{
+    if (dtype == FFTB_F32) return kind == K_C2R && k.nf >= 1792;
+    if (k.plan.S < 2 || (kind == K_R2C && !half)) return false;
+    return k.nf < (kind == K_R2C || kind == K_C2R ? 48 : 64);
+}
+
 int program_add(Program &prog, int dtype, const AxisPass &p)
 {
     if (p.n < 1) return FFTB_ERROR_INVALID_VALUE;
@@ -417,11 +434,13 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
     if (line) {
         // the thread mapping follows the input side; a side of the other order, or with blocked
         // points, is staged through shared memory
-        const LineKernelInfo &k = *r.find_line(dtype, nf, a.in_pts_fast ? 1 : 0);
+        const bool row = a.in_pts_fast &&
+                         (a.out_pts_fast || !columns_from_rows(dtype, p.kind, half, *r.find_line(dtype, nf, 1)));
+        const LineKernelInfo &k = *r.find_line(dtype, nf, row ? 1 : 0);
         if ((p.ep_mode & ~(EP_SCALE | EP_HALFW | EP_TWIDDLE | EP_DERIV)) != 0 && p.kind != K_SANDWICH) return FFTB_ERROR_INVALID_VALUE;
         L.line = &k;
-        a.line_in = !p.in_blk && (!k.row || p.is == 1);
-        a.line_out = a.out_pts_fast == a.in_pts_fast && !p.out_blk && (!k.row || p.os == 1);
+        a.line_in = !p.in_blk && (row ? p.is == 1 : !a.in_pts_fast);
+        a.line_out = !p.out_blk && (row ? p.os == 1 : !a.out_pts_fast);
         line_divisors(a);
         void *tab = nullptr;
         if ((st = get_stages(dtype, k, &tab)) != FFTB_SUCCESS) return st;

@@ -183,3 +183,36 @@ def test_short_double_columns_are_as_fast_as_a_copy_allows(F, torch_cuda):
         lines = (1 << 22) // n
         plan = F.Plan(F.C2CF, [n], [n], lines, 1, [n], lines, 1, lines, dtype="float64")
         assert us(lambda: plan.exec(x, y)) <= 2 * copy, n
+
+
+# from rows to columns, on both sides of the lengths where the mapping changes (double: 4 and more split
+# points up to 63, real lines up to 94; float C2R: 3584 points and more), a last tile that is not full
+MIXED = [("float64", k, n) for k, ns in (("F", (2, 3, 4, 8, 35, 63, 64)), ("I", (4, 13, 60, 64)),
+                                         ("R", (4, 6, 8, 16, 35, 90, 94, 96, 98)),
+                                         ("C", (4, 6, 8, 16, 35, 45, 47, 49, 90, 96, 98))) for n in ns]
+MIXED += [("float32", "C", n) for n in (3456, 3500, 3584, 3600, 3840, 4096, 8192)]
+
+
+@pytest.mark.parametrize("dtype,kind,n", MIXED)
+def test_rows_to_columns(F, torch_cuda, dtype, kind, n):
+    torch = torch_cuda
+    rng = np.random.default_rng(n)
+    lines, h = (331, n // 2 + 1) if n < 100 else (13, n // 2 + 1)
+    real, comp = (np.float32, np.complex64) if dtype == "float32" else (np.float64, np.complex128)
+    u = rng.uniform(-1, 1, (lines, n)).astype(real)
+    z = (u + 1j * rng.uniform(-1, 1, (lines, n))).astype(comp)
+    half = np.fft.rfft(u.astype(np.float64))
+    x, ref, d, ni, no = {"F": (z, np.fft.fft(z), F.C2CF, n, n),
+                         "I": (z, np.fft.ifft(z) * n, F.C2CB, n, n),
+                         "R": (u, half, F.R2C, n, h),
+                         "C": (half.astype(comp), u.astype(np.float64) * n, F.C2R, h, n)}[kind]
+    out_type = getattr(torch, str(np.dtype(real if kind == "C" else comp)))
+    # three points of room behind every line and three lines of room between the rows of the output
+    pad = np.full((lines, ni + 3), 1e30, x.dtype)
+    pad[:, :ni] = x
+    out = torch.full((no, lines + 3), 7.0, dtype=out_type, device="cuda")
+    plan = F.Plan(d, [n], [ni], 1, ni + 3, [no], lines + 3, 1, lines, dtype=dtype)
+    plan.exec(torch.from_numpy(pad).cuda(), out)
+    got = out.cpu().numpy()
+    assert rel(got[:, :lines].T, ref) <= TOL[dtype]
+    assert (got[:, lines:] == 7.0).all()
