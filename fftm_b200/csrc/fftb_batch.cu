@@ -406,7 +406,7 @@ int build_plan(fftb_batch_s *b, int op, double sign)
         const Launch &L = P.seq.launches[p];
         PassArgs a = L.args;
         // line tiles of 256 threads; chirp-z, long and other lengths: sequential only
-        const bool tiled = batch_nf_supported(L.k.nf) && L.line && a.line_in && a.line_out &&
+        const bool tiled = batch_nf_supported(L.nf) && L.line && a.line_in && a.line_out &&
                            !(L.line->row && a.kind == K_SANDWICH);
         if (!tiled) P.persistent_ok = false;
         const int G = L.line ? L.line->G : a.G;
@@ -420,23 +420,23 @@ int build_plan(fftb_batch_s *b, int op, double sign)
         pb.out_buf = L.out_buf;
         pb.in_off = (long long)L.in_off_bytes;
         pb.out_off = (long long)L.out_off_bytes;
-        pb.nf = L.k.nf;
+        pb.nf = L.nf;
         pb.lkind = a.kind == K_SANDWICH ? 2 : (L.line && L.line->row ? 0 : 1);
         ntiles[p] = (int)((a.nlines + G - 1) / G);
         // the row-pair tile, where it is the faster one (row_group_tile_pairs)
         const int st = stage_of[p], ti = trans_of[p];
-        const int FZ = st_zdir[st] >= 0 ? row_group_tile_pairs(b->dtype, 2 * L.k.nf) : 0;
+        const int FZ = st_zdir[st] >= 0 ? row_group_tile_pairs(b->dtype, 2 * L.nf) : 0;
         if (FZ > 0) {
             // its set-up (shared-memory limit, root table) once per direction and length
-            void *&roots = roots_of[st_zdir[st] * 100000 + 2 * L.k.nf];
+            void *&roots = roots_of[st_zdir[st] * 100000 + 2 * L.nf];
             if (!roots) {
-                int rs = row_group_prepare(b->dtype, st_zdir[st], 2 * L.k.nf, &roots);
+                int rs = row_group_prepare(b->dtype, st_zdir[st], 2 * L.nf, &roots);
                 if (rs != FFTB_SUCCESS) return rs;
             }
             const long long rows = b->dims[3 * ti] * b->dims[3 * ti + 1];
             pb.pair = 1;
             pb.dir = st_zdir[st];
-            pb.n = 2 * L.k.nf;
+            pb.n = 2 * L.nf;
             pb.lines = (int)rows;
             pb.scale = st_zdir[st] == 1 && (a.ep_mode & EP_SCALE) ? (float)a.ep_scale : 1.0f;
             pb.roots = (const float2 *)roots;

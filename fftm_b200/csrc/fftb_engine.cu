@@ -275,18 +275,17 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
         return FFTB_ERROR_UNSUPPORTED_SIZE;
     }
     bool chirpz = false;
-    if (line) {
-        if (!lookup_kernel(nf, &L.k)) L.k = PassKernelInfo{nf, 1, pad16(nf) + 1, nullptr};
-    } else if (bluestein_kernel(dtype, p.n, &L.k)) {
-        chirpz = true;   // L.k.nf is the convolution length
+    PassKernelInfo bs = {};  // the chirp-z pass; bs.nf is its convolution length
+    if (!line && bluestein_kernel(dtype, p.n, &bs)) {
+        chirpz = true;
         const void *ch = nullptr, *bh = nullptr;
         int st = bluestein_tables(dtype, p.n, &ch, &bh);
         if (st != FFTB_SUCCESS) return st;
         a.bs_n = p.n;
         a.bs_chirp = ch;
         a.bs_bhat = bh;
-    } else {
-        // longer than one pass kernel holds: a long-line step (four-step or chirp-z)
+    } else if (!line) {
+        // longer than one pass holds: a long-line step (four-step or chirp-z)
         if (p.in_blk || p.out_blk) {
             set_last_error("blocked point indices need a C2C pass kernel (line length up to 4096)");
             return FFTB_ERROR_UNSUPPORTED_SIZE;
@@ -296,6 +295,7 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
         if (st != FFTB_SUCCESS) return st;
         Launch S;
         memset(&S.args, 0, sizeof(S.args));
+        S.nf = 0;
         S.fn = nullptr;
         S.line = nullptr;
         S.programmatic = 0;
@@ -317,7 +317,8 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
         prog.launches.push_back(S);
         return FFTB_SUCCESS;
     }
-    const int ntw = chirpz ? L.k.nf : (half ? 2 * nf : nf);
+    L.nf = chirpz ? bs.nf : nf;
+    const int ntw = half ? 2 * nf : L.nf;
     void *roots = nullptr;
     int st = get_roots(dtype, ntw, &roots);
     if (st != FFTB_SUCCESS) return st;
@@ -360,7 +361,6 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
     a.out_blk = p.out_blk;
     a.out_hi = p.out_hi;
     const size_t cb = complex_bytes(dtype);
-    a.tw_smem = ((size_t)ntw * cb <= 16384) ? 1 : 0;
 
     // epilogue
     a.ep_mode = p.ep_mode;
@@ -405,30 +405,7 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
     }
     L.real_align = 2 * real_bytes(dtype);
 
-    // lines per CTA
-    const int T = L.k.threads_per_line;
-    int G = std::max(1, 256 / T);
-    if (!a.in_pts_fast || !a.out_pts_fast) G = std::max(G, 16);
-    G = std::min(G, std::max(1, 512 / T));
-    G = floor_pow2(G);
-    const long long lines_pow2 = nlines;
-    while (G > 1 && G / 2 >= lines_pow2) G /= 2;
-    auto smem_of = [&](int g) -> size_t {
-        return (a.tw_smem ? (size_t)ntw * cb : 0) + (size_t)g * 32 + (size_t)g * (size_t)L.k.line_pitch * cb;
-    };
-    while (G > 1 && smem_of(G) > 160 * 1024) G /= 2;
-    if (smem_of(G) > 227 * 1024) {
-        set_last_error("line too long for shared memory");
-        return FFTB_ERROR_UNSUPPORTED_SIZE;
-    }
-    a.G = G;
-    int gs = 0;
-    while ((1 << gs) < G) ++gs;
-    a.gshift = gs;
-    L.block = G * T;
-    L.smem = smem_of(G);
-    long long ncta = (nlines + G - 1) / G;
-    L.fn = L.k.fn;
+    long long ncta = 0;
     L.line = nullptr;
     L.programmatic = line ? 1 : 0;
     if (line) {
@@ -449,6 +426,28 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
         L.block = k.NT;
         L.smem = a.line_in && a.line_out ? k.smem : k.smem_t;
         ncta = (nlines + k.G - 1) / k.G;
+    } else {
+        // chirp-z: lines per CTA
+        const int T = bs.threads_per_line;
+        a.tw_smem = ((size_t)ntw * cb <= 16384) ? 1 : 0;
+        int G = std::max(1, 256 / T);
+        if (!a.in_pts_fast || !a.out_pts_fast) G = std::max(G, 16);
+        G = floor_pow2(std::min(G, std::max(1, 512 / T)));
+        while (G > 1 && G / 2 >= nlines) G /= 2;
+        auto smem_of = [&](int g) -> size_t {
+            return (a.tw_smem ? (size_t)ntw * cb : 0) + (size_t)g * 32 + (size_t)g * (size_t)bs.line_pitch * cb;
+        };
+        while (G > 1 && smem_of(G) > 160 * 1024) G /= 2;
+        if (smem_of(G) > 227 * 1024) {
+            set_last_error("line too long for shared memory");
+            return FFTB_ERROR_UNSUPPORTED_SIZE;
+        }
+        a.G = G;
+        while ((1 << a.gshift) < G) ++a.gshift;
+        L.fn = bs.fn;
+        L.block = G * T;
+        L.smem = smem_of(G);
+        ncta = (nlines + G - 1) / G;
     }
     if (ncta > 0x7fffffffLL) return FFTB_ERROR_INVALID_VALUE;
     L.grid = dim3((unsigned)ncta, 1, 1);
@@ -482,7 +481,7 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
         const long long pout = (p.kind == K_R2C) ? (long long)(p.n / 2 + 1) : (long long)p.n;
         L.alg_bytes = (double)nlines * ((double)pin * (double)in_el + (double)pout * (double)out_el);
         L.name = std::string(chirpz ? "fftb_bluestein_kernel<" : "fftb_line_kernel<") + (dtype == 0 ? "f32" : "f64") +
-                 "," + std::to_string(chirpz ? L.k.nf : nf) + ">/" + kn[p.kind] + "/n" + std::to_string(p.n);
+                 "," + std::to_string(L.nf) + ">/" + kn[p.kind] + "/n" + std::to_string(p.n);
     }
     prog.dtype = dtype;
     prog.launches.push_back(L);

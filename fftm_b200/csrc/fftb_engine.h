@@ -58,7 +58,7 @@ struct LineKernelInfo;
 
 struct Launch {
     PassArgs args;
-    PassKernelInfo k;    // the pass kernel's tile of this length (the batch kernels run it)
+    int nf;              // complex length of the kernel's lines (chirp-z: its convolution length)
     const void *fn;      // the kernel this launch runs: the line kernel, or the chirp-z pass
     const LineKernelInfo *line;  // its line kernel (null: chirp-z or a long-line step)
     int programmatic;    // fn waits for its predecessor itself (programmatic launch)

@@ -936,7 +936,9 @@ template <typename R, int N, bool ROW> inline LineKernelInfo line_kernel_info()
     k.G = S::G;
     k.NT = S::NT;
     k.smem = sizeof(cpx<R>) * S::EX;
-    k.smem_t = sizeof(cpx<R>) * (S::EX > S::ST ? S::EX : S::ST);
+    constexpr size_t staged = sizeof(cpx<R>) * (S::EX > S::ST ? S::EX : S::ST);
+    static_assert(staged + S::G * sizeof(long long) + 1024 <= 228 * 1024, "a CTA's shared memory, its line offsets and 1 KB of the system's");
+    k.smem_t = staged;
     k.plan = S::P;
     k.fn = (const void *)&fftb_line_kernel<R, N, ROW, false>;
     k.fn_sand = (const void *)&fftb_line_kernel<R, N, ROW, true>;
