@@ -332,6 +332,15 @@ int build_derivative(fftb_ffts_s *o)
     const int d = o->dtype, ih = o->dim - 1;  // the half axis is the last one
     const long long len[4] = {nx, ny, nz, nw};
     const long long nh = len[ih], nhh = nh / 2 + 1;
+    // every axis needs a line kernel: asked first, because a long-line step that is built takes its work
+    // lines at once
+    for (int ax = 0; ax < o->dim; ++ax) {
+        const bool packed = ax == ih && nh % 2 == 0 && has_kernel(d, (int)(nh / 2));
+        if (!packed && !has_kernel(d, (int)len[ax])) {
+            o->drv = -1;
+            return FFTB_SUCCESS;
+        }
+    }
     // strides of the axes in the real array and in S, slowest to fastest x, y, (z, w), or w, z, y, x
     long long rs[4], ss[4], r = 1, sp = 1;
     const bool pencil = o->dim == 4 && o->layout == FFTB_4D_PENCIL;
@@ -363,12 +372,8 @@ int build_derivative(fftb_ffts_s *o)
     if (st == FFTB_SUCCESS) st = add(o->drv_half, K_C2R, ih, EP_SCALE | EP_DERIV, 1.0 / (double)nh);
     for (int ax = 0; ax < ih && st == FFTB_SUCCESS; ++ax)
         st = add(o->drv_axis[ax], K_SANDWICH, ax, EP_SCALE | EP_DERIV, 1.0 / (double)len[ax]);
-    if (st == FFTB_ERROR_UNSUPPORTED_SIZE) {  // a chirp-z or long axis
-        o->drv = -1;
-        return FFTB_SUCCESS;
-    }
     if (st == FFTB_SUCCESS) o->drv = 1;
-    return st;
+    return st == FFTB_ERROR_ALLOC ? FFTB_SUCCESS : st;  // no memory for a table: the whole transform, this time
 }
 
 bool aligned16(const void *a, const void *b) { return ((uintptr_t)a % 16 == 0) && ((uintptr_t)b % 16 == 0); }

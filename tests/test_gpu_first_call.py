@@ -41,3 +41,27 @@ def test_first_use_of_a_length(F):
     out = subprocess.run([sys.executable, "-c", FIRST_USE], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert out.returncode == 0, out.stderr
     assert float(out.stdout.split()[-1]) < 0.012
+
+
+def test_first_derivative_keeps_only_its_spectra(F, torch_cuda):
+    """An object with a length that has no line kernel takes the whole transform for its derivatives: the
+    first call keeps the spectrum buffers and no work lines (two of 64 MB each for the R2C, and for the
+    C2R, of a 10007-point axis)."""
+    torch = torch_cuda
+    dims = (16, 16, 10007)
+    x = torch.randn(dims, device="cuda")
+    outs = [torch.empty_like(x) for _ in dims]
+
+    def kept():
+        f = F.ffts("float32").init(*dims)
+        gc.collect()
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        f.derivative(x, outs[0], 0)
+        f.gradient(x, outs)
+        torch.cuda.synchronize()
+        return before - torch.cuda.mem_get_info()[0]
+
+    kept()  # what the process loads once
+    spectra = 2 * 16 * 16 * (10007 // 2 + 1) * 8
+    assert kept() <= spectra + 8 * 2 ** 20
