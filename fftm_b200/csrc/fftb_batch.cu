@@ -44,7 +44,6 @@
 namespace fftb {
 namespace {
 
-constexpr int kBatchThreads = 256;
 constexpr long long kSpinLimit = 1LL << 22;  // ~0.5 s of polling at most
 
 struct BatchItem {
@@ -93,7 +92,6 @@ template <int NF, int LKIND>
 __device__ __noinline__ void batch_tile(const PassArgs *a, const void *in, void *out, long long tile,
                                         unsigned char *smem)
 {
-    static_assert(LineShape<float, NF, LKIND == 0>::NT <= kBatchThreads, "a tile fits the batch kernels' blocks");
     line_body<float, NF, LKIND == 0, LKIND == 2, true>(*a, in, out, tile, smem, nullptr);
 }
 
@@ -376,7 +374,7 @@ int build_plan(fftb_batch_s *b, int op, double sign)
     }
     P.nstages = (int)tpass[0].size();
     P.npasses = (int)P.seq.launches.size();
-    // persistent form: the same passes with G capped to kBatchThreads threads per tile
+    // the one-launch forms: the same passes as tiles of kBatchThreads threads
     P.persistent_ok = (b->dtype == FFTB_F32);
     std::vector<PassArgs> args(P.npasses);
     std::vector<PassBind> binds(P.npasses);
@@ -409,7 +407,7 @@ int build_plan(fftb_batch_s *b, int op, double sign)
         const bool tiled = batch_nf_supported(L.nf) && L.line && a.line_in && a.line_out &&
                            !(L.line->row && a.kind == K_SANDWICH);
         if (!tiled) P.persistent_ok = false;
-        const int G = L.line ? L.line->G : a.G;
+        const int G = L.line ? L.line->G : std::max(1, a.G);
         a.pair_io = L.pair_candidate ? 1 : 0;  // buffers are 16-byte aligned (checked at execution)
         const size_t sm = L.line ? L.line->smem : 0;
         smem = std::max(smem, sm);
@@ -493,16 +491,18 @@ int build_plan(fftb_batch_s *b, int op, double sign)
                 if (g.count > 0) P.groups.push_back(g);
                 continue;
             }
-            OpPlan::Group g{(int)gitems.size(), 0, nf, 0};
-            for (int i = 0; i < b->count; ++i) {
-                const int p = tpass[i][s];
-                if (binds[p].nf != nf) continue;
-                g.smem = std::max(g.smem, pass_smem[p]);
-                for (int t = 0; t < ntiles[p]; ++t) gitems.push_back(BatchItem{p, t});
+            for (int lkind = 0; lkind < 3; ++lkind) {  // a group is one kernel
+                OpPlan::Group g{(int)gitems.size(), 0, nf, 0};
+                g.lkind = lkind;
+                for (int i = 0; i < b->count; ++i) {
+                    const int p = tpass[i][s];
+                    if (binds[p].nf != nf || binds[p].lkind != lkind) continue;
+                    g.smem = std::max(g.smem, pass_smem[p]);
+                    for (int t = 0; t < ntiles[p]; ++t) gitems.push_back(BatchItem{p, t});
+                }
+                g.count = (int)gitems.size() - g.offset;
+                if (g.count > 0) P.groups.push_back(g);
             }
-            g.lkind = binds[gitems[g.offset].pass].lkind;
-            g.count = (int)gitems.size() - g.offset;
-            if (g.count > 0) P.groups.push_back(g);
         }
     }
     if (P.persistent_ok) {

@@ -193,6 +193,8 @@ __host__ __device__ constexpr int line_conflicts(const LinePlan &p, int n, int T
     return c;
 }
 
+constexpr int kBatchThreads = 256;  // threads of a batch kernel's block, whatever its tiles need
+
 constexpr int kLineEmax = 16;  // 16 complex values: 32 (float) or 64 (double) registers (radices above take more)
 
 template <typename R, int N, bool ROW> struct LineShape {
@@ -580,8 +582,10 @@ __device__ __forceinline__ void line_body(const PassArgs &__restrict__ a, const 
     // the last stage's radix (the sandwich ends with the reversed plan's last, r_0)
     constexpr int RL = SAND ? P.r[0] : P.r[P.S - 1], NBL = N / RL, PERL = (NBL + T - 1) / T;
     constexpr int PH = (N / 2 + T) / T;  // pairs (k, N - k), k = t + T i <= N/2, of a thread
-    // an extra thread repeats another's exchange writes, which only block-wide barriers order
-    static_assert(!BATCH || !S::WARP || NT == 256, "whole tiles where a warp orders its own exchanges");
+    // an extra thread takes the place of thread tid - NT, which has to be one of the tile; it repeats that
+    // thread's exchange writes, which only block-wide barriers order
+    static_assert(!BATCH || (NT <= kBatchThreads && 2 * NT >= kBatchThreads), "extra threads stay in the tile");
+    static_assert(!BATCH || !S::WARP || NT == kBatchThreads, "whole tiles where a warp orders its own exchanges");
     C *s = reinterpret_cast<C *>(smem_raw);
     const int tid = BATCH && threadIdx.x >= NT ? threadIdx.x - NT : threadIdx.x;
     const int g = ROW ? tid / T : tid % G, t = ROW ? tid - g * T : tid / G;
