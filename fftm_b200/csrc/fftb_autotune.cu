@@ -683,23 +683,21 @@ int measure_batch(fftb_batch b, int op, double sign, int warmup, int iters, Conf
         cands.push_back(c);
     }
     if (dtype == FFTB_F32) {
-        for (int ts : {1, 2})
-            for (int cps : {0, 1, 2}) {
-                Candidate c;
-                c.name = "graph-t" + std::to_string(ts) + "-c" + std::to_string(cps);
-                c.a = 2;
-                c.b = ts;
-                c.c = cps;
-                cands.push_back(c);
-            }
-        for (int ts : {1, 2}) {
+        // (the tiles have one size: tiles_scale stays 1)
+        for (int cps : {0, 1, 2}) {
             Candidate c;
-            c.name = "grouped-graph-t" + std::to_string(ts);
-            c.a = 4;
-            c.b = ts;
-            c.c = 0;
+            c.name = "graph-t1-c" + std::to_string(cps);
+            c.a = 2;
+            c.b = 1;
+            c.c = cps;
             cands.push_back(c);
         }
+        Candidate c;
+        c.name = "grouped-graph-t1";
+        c.a = 4;
+        c.b = 1;
+        c.c = 0;
+        cands.push_back(c);
     }
     const bool in_spec = op == FFTB_BATCH_BACKWARD, out_spec = op == FFTB_BATCH_FORWARD;
     const size_t nin = in_spec ? (size_t)stot * 2 : (size_t)rtot;     // reals

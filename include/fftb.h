@@ -332,9 +332,10 @@ int fftb_autotune_ffts(int dtype, long long nx, long long ny, long long nz, long
 /* Applies the FFTB_AUTOTUNE_STRATEGY / _PLANE_CLUSTER of a config to an ffts object. */
 int fftb_ffts_apply_config(fftb_ffts obj, const char *text);
 /* load_or_measure for a batch and one op: candidates are sequential launches, the
- * graph-replayed persistent launch with tiles_scale {1, 2} x ctas_per_sm {0, 1, 2}, and
- * the graph-replayed grouped launches with tiles_scale {1, 2}.  The winner's knobs are
- * applied to the batch and its mode returned in *mode. */
+ * graph-replayed persistent launch with ctas_per_sm {0, 1, 2}, and the graph-replayed grouped
+ * launches.  The winner's knobs are applied to the batch and its mode returned in *mode.
+ * (A cache that names tiles_scale 2, from before the tiles had one size, is accepted and runs
+ * the same.) */
 int fftb_autotune_batch(fftb_batch batch, int op, double sign, const char *cache_file, int flags, int warmup,
                         int iterations, char *text, size_t capacity, size_t *needed, int *from_cache, int *mode);
 /* Applies FFTB_AUTOTUNE_TILES_SCALE / _CTAS_PER_SM of a config; *mode = FFTB_AUTOTUNE_BATCH_MODE. */

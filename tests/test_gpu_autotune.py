@@ -207,3 +207,24 @@ def test_batch_autotune(F, torch_cuda, tmp_path):
     assert b2.autotune(B.ROUNDTRIP, path).source == "cache" and b2.mode == b.mode
     with pytest.raises(FftbError):
         B.Batch(shapes[:47]).autotune(B.ROUNDTRIP, path)
+
+
+def test_batch_candidates_are_distinct_forms(F, torch_cuda, tmp_path):
+    """No form is timed twice under two names, and a cache from when the tiles had two sizes still
+    applies."""
+    torch = torch_cuda
+    import fftm_b200.batch as B
+    b = B.Batch(B.draw_shapes(8, seed=4))
+    path = tmp_path / "batch.env"
+    b.autotune(B.ROUNDTRIP, path, measured=F.autotune.measured_options(warmup=1, iterations=1))
+    cfg = F.autotune.load_key_value_file(path)
+    assert cfg["FFTB_AUTOTUNE_CANDIDATES"].split(",") == ["sequential", "graph-t1-c0", "graph-t1-c1", "graph-t1-c2",
+                                                          "grouped-graph-t1"]
+    old = dict(cfg, FFTB_AUTOTUNE_BATCH_MODE="2", FFTB_AUTOTUNE_TILES_SCALE="2", FFTB_AUTOTUNE_CTAS_PER_SM="1",
+               FFTM_AUTOTUNE_STRATEGY_3D="graph-t2-c1")
+    assert b.apply_config(old) == 2
+    x = torch.rand(b.real_total, device="cuda")
+    out = torch.zeros_like(x)
+    b.exec(B.ROUNDTRIP, x, out)
+    assert b.status(B.ROUNDTRIP) == 0
+    assert float(torch.linalg.norm(out - x) / torch.linalg.norm(x)) <= 2e-6
