@@ -78,7 +78,7 @@ def profile_case(a) -> int:
 
       python bench.py --profile-case poisson3d --n 256 --reps 3      # fused 3D Poisson solve
       python bench.py --profile-case poisson3d --n 256 --cluster 4   # 4-CTA plane clusters
-      python bench.py --profile-case staged3d --n 256 --reps 3       # one pass kernel per axis
+      python bench.py --profile-case staged3d --n 256 --reps 3       # one line kernel per axis
       python bench.py --profile-case roundtrip4d --n 64 --reps 3     # 4D R2C + normalised C2R
       python bench.py --profile-case batch --count 512 --reps 2      # batched round trips
     """

@@ -491,7 +491,7 @@ class ffts:
     def set_strategy(self, strategy="auto", plane_cluster=0):
         """"auto", "fused" (multi-axis kernels; plane_cluster 1, 2, 4 or 8 CTAs per 3D
         plane, 0 by occupancy), "fused_tc" (fused, with the column kernels' first radix-16
-        stage on the tensor cores in split FP16) or "staged" (one pass kernel per axis)."""
+        stage on the tensor cores in split FP16) or "staged" (one kernel per axis)."""
         self._ensure()
         code = {"auto": 0, "fused": 1, "staged": 2, "fused_tc": 3}[strategy]
         _check(_lib.load().fftb_ffts_set_strategy(self._h, code, int(plane_cluster)), "set_strategy")

@@ -287,7 +287,7 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
     } else if (!line) {
         // longer than one pass holds: a long-line step (four-step or chirp-z)
         if (p.in_blk || p.out_blk) {
-            set_last_error("blocked point indices need a C2C pass kernel (line length up to 4096)");
+            set_last_error("blocked point indices need a C2C line kernel (line length up to 4096)");
             return FFTB_ERROR_UNSUPPORTED_SIZE;
         }
         std::shared_ptr<LongLine> ll;
@@ -353,7 +353,7 @@ int program_add(Program &prog, int dtype, const AxisPass &p)
     a.ep_tw = p.ep_tw;
     if ((p.in_blk || p.out_blk) && (chirpz || (p.kind != K_C2C_FWD && p.kind != K_C2C_INV) ||
                                     (p.out_blk && p.n / p.out_blk > 8))) {
-        set_last_error("blocked point indices need a C2C pass kernel and at most 8 blocks");
+        set_last_error("blocked point indices need a C2C line kernel and at most 8 blocks");
         return FFTB_ERROR_UNSUPPORTED_SIZE;
     }
     a.in_blk = p.in_blk;

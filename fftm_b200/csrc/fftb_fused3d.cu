@@ -1036,7 +1036,6 @@ namespace {
 const void *row_group_fn(int dir, int nz)
 {
     switch (nz) {
-    case 32: return dir ? (const void *)&row_group_kernel<32, 1> : (const void *)&row_group_kernel<32, 0>;
     case 64: return dir ? (const void *)&row_group_kernel<64, 1> : (const void *)&row_group_kernel<64, 0>;
     case 128: return dir ? (const void *)&row_group_kernel<128, 1> : (const void *)&row_group_kernel<128, 0>;
     case 256: return dir ? (const void *)&row_group_kernel<256, 1> : (const void *)&row_group_kernel<256, 0>;

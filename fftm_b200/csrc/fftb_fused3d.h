@@ -38,7 +38,7 @@ int fused3d_forward_adjoint(const Fused3D &f, void *gspec, void *greal, cudaStre
 int fused3d_backward_adjoint(const Fused3D &f, const void *greal, void *gspec, cudaStream_t s, LaunchTimer *t);
 int fused3d_num_launches(const Fused3D &f, int which);
 
-// The z stage of many f32 3D transforms of one z length (32-256, a power of two) in one launch:
+// The z stage of many f32 3D transforms of one z length (64-256, a power of two) in one launch:
 // R2C (dir 0) or scaled C2R (dir 1) of two contiguous real rows per complex FFT.
 struct RowGroupItem {
     long long roff;  // floats from the real buffer base to the transform's rows [nrows][nz]

@@ -3,13 +3,13 @@
 // Bound: memory.  A pass reads every line once and writes it once, so the kernel keeps a line in
 // registers from its load to its store: the first butterfly's points come straight from global
 // memory into the registers that transform them, the last butterfly's results are stored
-// straight from registers, and shared memory carries only the exchanges between the two or
-// three stages (S - 1 of them for S stages).  Every thread issues all of its line's loads before it
+// straight from registers, and shared memory carries only the exchanges between the stages
+// (S - 1 of them; up to 4096 points S is at most five, and two or three for most lengths).  Every thread issues all of its line's loads before it
 // waits for the first, which is what keeps enough bytes in flight.  Per launch, bytes read and
 // written over the time on a B200, this kernel and the pass kernel it replaced (fftb_pass.cuh: all
-// points through shared memory before and after the transform): 512^3 f32 R2C 165 us = 6.5 TB/s
-// (406 us), x or y C2C 235 us = 4.6 TB/s (533 us), x sandwich 336 us (1118 us); 256^3 f64 C2C
-// 49-55 us = 5.0-5.5 TB/s (74-82 us); 192^3 f32 C2C 16.4 us (30.7 us).
+// points through shared memory before and after the transform): 512^3 f32 R2C 172 us = 6.2 TB/s
+// (406 us), x or y C2C 215 us = 5.0 TB/s (533 us), x sandwich 305 us (1118 us); 256^3 f64 C2C
+// 51-53 us = 5.1-5.3 TB/s (74-82 us); 192^3 f32 C2C 16.4 us (30.7 us).
 //
 // Lines are n = r_0 r_1 ... points (Stockham order: Govindaraju et al., "High performance
 // discrete Fourier transforms on graphics processors", SC 2008); the plan takes the fewest
@@ -201,9 +201,9 @@ template <typename R, int N, bool ROW> struct LineShape {
     static constexpr LinePlan P = line_plan(N, ROW, kLineEmax, sizeof(R) == 4 ? 32 : 16);
     static constexpr LinePlan Q = line_reverse(P);
     static constexpr int T = P.T, E = P.E;
-    // lines per CTA.  ROW: as near to 256 threads as fills its warps best.  COL: segments of at
-    // least 64 bytes (8 float, 4 double lines) and 256 threads, up to 1024 threads and 160 KB of
-    // exchange area (512^3 f32 Poisson back to back: 1113 us with 64-byte segments, 1137 with 128).
+    // lines per CTA.  ROW: as near to 256 threads as fills its warps best.  COL: 256 threads, and
+    // segments of 64 bytes (8 float, 4 double lines) where 1024 threads and 160 KB of exchange area
+    // allow them (float columns of 1500, 2000 and 4096 points get 32 bytes, 2401 and 3000 points 16) (512^3 f32 Poisson back to back: 1113 us with 64-byte segments, 1137 with 128).
     // Double lines of one thread: past 32 lines while the tile is below 6 KB, because a CTA of one warp
     // with a few values a thread is bound by CTA starts (2^22 points as C2C columns of 1, 2 and 4
     // points 136 -> 36, 69 -> 25 and 35 -> 22 us, R2C of 4, 8 and 16 points 35 -> 13, 18 -> 11 and
@@ -402,7 +402,6 @@ template <typename R, typename C> __device__ __forceinline__ void dft9(C *v)
     }
 }
 
-// forward DFT of RAD values in registers
 // A x B with the twiddles w_AB^(n k) between
 template <typename R, int A, int B, typename C> __device__ __forceinline__ void dft_ct(C *v)
 {
@@ -427,6 +426,7 @@ template <typename R, int A, int B, typename C> __device__ __forceinline__ void 
     }
 }
 
+// forward DFT of RAD values in registers
 template <typename R, int RAD, typename C> __device__ __forceinline__ void line_dft(C *v)
 {
     if constexpr (RAD == 18) dft_pfa<R, 2, 9>(v);

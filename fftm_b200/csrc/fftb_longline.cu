@@ -1,4 +1,4 @@
-// fftb_longline.cu -- lines longer than one pass kernel holds in shared memory (more
+// fftb_longline.cu -- lines longer than one line kernel holds (more
 // than 4096 points, the reference's cuFFT plans accept any length,
 // source/external_wrap/fft_wrap_many.h:137-186).
 //
@@ -6,15 +6,15 @@
 //   gather   the input line into the work line (C2C: copied; R2C: real parts; C2R: the
 //            Hermitian extension of the half spectrum), zero padded to L;
 //   FFT_L    four-step: L = L1 * L2 with X[k1 + L1 k2] = sum_j2 w_L2^(j2 k2) w_L^(j2 k1)
-//            sum_j1 x[j2 + L2 j1] w_L1^(j1 k1), as two pass-engine passes over the work
+//            sum_j1 x[j2 + L2 j1] w_L1^(j1 k1), as two line-kernel passes over the work
 //            lines (length L1 with stride L2, the w_L^(j2 k1) twiddle fused into its
-//            store; then length L2), each factor a pass kernel of its own;
+//            store; then length L2), each factor a line kernel of its own;
 //   scatter  the work line to the output (C2C: all points; R2C: the half spectrum; C2R:
 //            the real parts), times the pass's epilogue factor (scale, Poisson, Gaussian,
-//            half-axis weights: the same rules as the pass kernel's store).
+//            half-axis weights: the same rules as the other passes').
 // A sandwich pass (forward FFT, spectral multiply, inverse FFT) runs FFT_L, the multiply,
 // and FFT_L^-1 on the work line.
-// When n has no split into two pass-kernel lengths (a large prime factor), the line runs
+// When n has no split into two line-kernel lengths (a large prime factor), the line runs
 // Bluestein's chirp-z (Bluestein 1970): L = M, a power of two >= 2n - 1; the gather
 // multiplies by the chirp c_j = exp(-i pi j^2 / n), FFT_M, a multiply by B = FFT_M(b) / M
 // with b the wrapped conj chirp (FP64 on the host), FFT_M^-1, and the scatter multiplies by
@@ -43,7 +43,7 @@ struct LongLine {
     int in_buf = B_IN, out_buf = B_OUT;
     size_t in_off = 0, out_off = 0;
     double scale = 1.0;
-    // epilogue, resolved as the pass kernel's (src 0: point index, 1..3: batch index b0..b2)
+    // epilogue, resolved as the other passes' (src 0: point index, 1..3: batch index b0..b2)
     int ep_mode = 0, ep_naxes = 0;
     int ep_src[4] = {0, 0, 0, 0}, ep_n[4] = {0, 0, 0, 0}, ep_half[4] = {0, 0, 0, 0};
     double ep_sign = -1.0, ep_gauss = 0.0, ep_hw = 1.0;
@@ -89,7 +89,7 @@ __device__ __forceinline__ long long line_off(long long l, const Geom &g, bool o
     return out ? b[0] * g.ob0 + b[1] * g.ob1 + b[2] * g.ob2 : b[0] * g.ib0 + b[1] * g.ib1 + b[2] * g.ib2;
 }
 
-// the pass kernel's epilogue factor (fftb_pass.cuh ep_factor) for point p of line l
+// the passes' epilogue factor for point p of line l
 template <typename R> __device__ R ll_factor(const Geom &g, int p, long long l)
 {
     long long b[3];
@@ -210,7 +210,7 @@ unsigned grid_for(long long total)
     return (unsigned)std::max(1LL, std::min(b, 148LL * 32));
 }
 
-// L1 * L2 = L with both factors pass-kernel lengths (not chirp-z), the split closest to
+// L1 * L2 = L with both factors line-kernel lengths (not chirp-z), the split closest to
 // the square root; 0 if none
 int split(int dtype, int L)
 {

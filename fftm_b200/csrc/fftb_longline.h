@@ -1,4 +1,4 @@
-// fftb_longline.h -- lines longer than the pass kernels hold in shared memory (internal).
+// fftb_longline.h -- lines longer than one line kernel or chirp-z pass holds (internal).
 #pragma once
 
 #include <memory>
@@ -10,7 +10,7 @@ namespace fftb {
 struct LongLine;
 
 // Builds the long-line step for pass `p` (C2C, R2C or C2R with at most a scale epilogue)
-// whose length no single pass kernel covers.  Returns FFTB_ERROR_UNSUPPORTED_SIZE when the
+// whose length no single kernel covers.  Returns FFTB_ERROR_UNSUPPORTED_SIZE when the
 // pass asks for something the long-line form does not do.
 int longline_create(int dtype, const AxisPass &p, std::shared_ptr<LongLine> &out);
 // Runs it with the program's buffers bound (in, out, work); ep: the dynamic scale, if any.

@@ -11,7 +11,7 @@
 // This entry point keeps its scratch -- the twiddle tables and the spectrum of
 // the solve -- in one file-scope __device__ array of fixed size, which every GPU
 // that loads the library holds until the process exits.  The kernels it runs are
-// the same pass kernels as the regular path (R2C on z, C2C on y, the x pass with
+// the pass kernels of fftb_pass.cuh (R2C on z, C2C on y, the x pass with
 // the -1/|k|^2 multiply between its forward and inverse FFT, C2C^-1 on y, C2R on
 // z with 1/N).
 #include <cuda_runtime.h>

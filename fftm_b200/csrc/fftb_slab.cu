@@ -3,7 +3,7 @@
 // (source/detail/mpi_transpose_3d_same_x.h for 3D, source/detail/mpi_transpose_4d_same_xw.h:
 // 437-497 for 4D) pack a send buffer, exchange, and unpack around the FFTs.  Here the pack is
 // the store of the last FFT pass before the exchange and the unpack the load of the first
-// FFT pass after it (blocked point indices, fftb_pass.cuh), so the exchange moves the
+// FFT pass after it (blocked point indices, fftb_line.cuh), so the exchange moves the
 // pass outputs as they are: one contiguous block per destination rank.  The exchange itself
 // is the caller's (an NCCL all-to-all, or nothing at all when the pack pass stores straight
 // into the peers' receive buffers through the pointer table of set_peers).

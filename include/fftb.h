@@ -80,10 +80,10 @@ typedef struct fftb_plan_s *fftb_plan;
  * batch) -> create_plan -> cufftMakePlanMany64 (source/external_wrap/cufft_wrap.h:533-566,
  * :1237-1259).  inembed/onembed may be NULL for the default tight layout
  * (cufft_wrap.h:568-587).  *work_bytes receives the work-area size (may be 0).
- * Line lengths: any length up to 4096 runs one pass kernel per axis (radix passes, or
+ * Line lengths: any length up to 4096 runs one kernel per axis (radix stages, or
  * chirp-z for a large prime factor); longer lines (up to 2^24 points, or 2^21 when a
  * prime factor above 4096 needs chirp-z) run a long-line step -- four-step through two
- * pass kernels, or chirp-z over a power-of-two four-step convolution -- that keeps two
+ * line kernels, or chirp-z over a power-of-two four-step convolution -- that keeps two
  * work lines of its own (lines x length complex values each) for the plan's lifetime. */
 int fftb_plan_create(int direction, int dtype, int rank, const long long *n, const long long *inembed,
                      long long istride, long long idist, const long long *onembed, long long ostride,
@@ -228,7 +228,7 @@ int fftb_ffts_timing_read(fftb_ffts obj, float *ms, double *bytes, char *names, 
  *          cluster size picked by occupancy; per-axis pass programs otherwise
  *  FUSED   fused kernels (FFTB_ERROR_UNSUPPORTED_SIZE when the size has none); for 3D,
  *          plane_cluster 1, 2, 4 or 8 picks the CTAs per (y, z) plane (0: by occupancy)
- *  STAGED  one pass kernel per axis (the generic pass programs)
+ *  STAGED  one line kernel (or chirp-z pass) per axis: the generic pass programs
  *  FUSED_TC  FUSED with the column kernels (3D: x; 4D: y and x) running their first
  *          radix-16 stage as a 16x16 complex contraction on the tensor cores in split
  *          FP16 (head + tail operands, FP32 accumulation); float32 only */

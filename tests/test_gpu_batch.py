@@ -55,9 +55,8 @@ def test_batch_forward_backward_vs_oracle(B, torch_cuda, mode):
         assert O.rel_l2(res[o:o + n], host[o:o + n].astype(np.float64)) <= TOL, (i, s)
 
 
-# lengths with and without the fused path's column and row tiles side by side in one stage
-# (x, y: 32-128 column tiles, 8-40 the pass kernel; z: 64-256 row tiles, 16-96 the pass
-# kernel), and spectra with fewer lines than one tile
+# line tiles of many lengths side by side in one stage (z rows of 64, 128 and 256 points in row-pair
+# tiles beside them), and spectra with fewer lines than one tile
 EDGE_SHAPES = [(8, 12, 64), (12, 8, 128), (32, 20, 64), (64, 12, 128), (48, 16, 96), (96, 32, 40), (16, 16, 256),
                (128, 8, 32), (20, 48, 128), (40, 96, 16)]
 
@@ -112,10 +111,9 @@ def test_batch_roundtrip_poisson_modes_agree(B, torch_cuda):
             torch.cuda.synchronize()
             assert b.status(op) == 0
             outs[(op, mode)] = out.cpu().numpy()
-        # the persistent and grouped modes run the same tiles (the fused path's column and
-        # z-row tiles where a stage has them), so they agree bit for bit; the sequential mode
-        # runs every stage on the pass kernel (half-length z FFTs, the Poisson multiply by a
-        # division) and agrees with them to rounding
+        # the persistent and grouped modes run the same tiles (the line kernel's, and row pairs for z
+        # rows of 64 points and more), so they agree bit for bit; the sequential mode runs
+        # every stage on the line kernel (half-length z FFTs) and agrees with them to rounding
         for mode in (2, 3, 4):
             np.testing.assert_array_equal(outs[(op, 1)], outs[(op, mode)])
         d = O.rel_l2(outs[(op, 1)].astype(np.float64), outs[(op, 0)].astype(np.float64))

@@ -1,6 +1,6 @@
 """GPU parity of lines longer than 4096 points (the reference's cuFFT plans take any
 length, source/external_wrap/fft_wrap_many.h:137-186): the four-step long-line step
-(n = L1 * L2, both pass-kernel lengths) and, for a large prime factor, chirp-z over a
+(n = L1 * L2, both line-kernel lengths) and, for a large prime factor, chirp-z over a
 power-of-two four-step convolution.  1D C2C plans both ways and R2C / C2R plans against
 numpy's FP64 FFT, strided batches, and 3D ffts with a long axis against the FP64 oracle.
 Tolerances: 2e-6 (f32) for the four-step form; the chirp-z form in f32 carries the

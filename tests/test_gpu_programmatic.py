@@ -126,6 +126,51 @@ def test_captured_calls(F, torch_cuda, dims, layout, dtype):
         _check(torch, *xs, layout, dtype)
 
 
+@pytest.mark.parametrize("dims,layout,dtype", [CASES[0], CASES[3], CASES[6], CASES[8]])
+def test_captured_among_other_work(F, torch_cuda, dims, layout, dtype):
+    """Captured behind and between a kernel, a copy and a memset of torch's, and behind a join of two
+    streams (a launch with two predecessors): the edges to those are full ones."""
+    torch = torch_cuda
+    real, comp = _types(torch, dtype)
+    f = _object(F, torch, dims, layout, dtype)
+    x = torch.zeros(dims, dtype=real, device="cuda")
+    x2, back, sol = (torch.empty_like(x) for _ in range(3))
+    spec, kept = (torch.empty(f.spectrum_shape(), dtype=comp, device="cuda") for _ in range(2))
+    side = torch.cuda.Stream()
+
+    def calls():
+        main = torch.cuda.current_stream()
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            sol.mul_(0)              # a kernel beside ...
+        torch.mul(x, 2, out=x2)      # ... a kernel
+        main.wait_stream(side)
+        f.forward(x2, spec)          # two predecessors
+        kept.copy_(spec)             # a copy
+        f.backward(spec, back, normalized=True)
+        spec.zero_()                 # a memset
+        f.poisson(x2, sol)
+        back.mul_(0.5)
+
+    warm = torch.cuda.Stream()
+    warm.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(warm):
+        calls()
+    warm.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        calls()
+    results = []
+    for _ in range(4):
+        x.copy_(torch.randn(dims, dtype=real, device="cuda"))
+        graph.replay()
+        graph.replay()
+        results.append([t.clone() for t in (x, kept, back, sol)])
+    torch.cuda.synchronize()
+    for xs, spectrum, b, u in results:
+        _check(torch, xs, spectrum / 2, b, u / 2, layout, dtype)
+
+
 def test_calls_follow_the_stream(F, torch_cuda):
     """One object and one plan used on two streams in turn: each call runs on the stream it is given or
     finds current, also when it is the stream of two calls ago, and when the handle was last used on
