@@ -189,12 +189,12 @@ def test_calls_follow_the_stream(F, torch_cuda):
     torch.cuda.synchronize()
 
     def on(stream, how):
-        """Runs both calls on `stream` while the other one is busy for about 50 ms."""
+        """Runs both calls on `stream` while the other one is busy for about 150 ms."""
         other = s2 if stream is s1 else s1
         a, b = torch.zeros_like(spec), torch.zeros_like(y)
         torch.cuda.synchronize()
         with torch.cuda.stream(other):
-            torch.cuda._sleep(100_000_000)
+            torch.cuda._sleep(300_000_000)
         if how == "argument":
             f.forward(x, a, stream=stream)
             plan.exec(z, b, stream=stream)
